@@ -14,6 +14,7 @@
 #include "topology.h"
 #include "cloth_internal.h"
 #include "grid_cg.cuh"
+#include "resident_cg.h"
 #include "broadphase_order.h"
 
 using namespace b3g;
@@ -123,10 +124,20 @@ b3g_status ensure_cg_rec(b3g_cloth* c)
 // cooperative launch (two grid reductions per iteration, or the fused form).
 cudaError_t launch_persistent_cg(b3g_cloth* c, int dot, cudaStream_t st)
 {
-    cudaError_t e = cudaMemsetAsync(c->dev.bar, 0, sizeof(GridBarrier), st);
+    const ResShape shape = c->cg_strategy == B3G_CG_PERSISTENT ? resident_shape(c->dev) : ResShape();
+    if (shape.ctas) return launch_resident_cg(c->dev, shape, dot, st);
+    cudaError_t e = cudaMemsetAsync(c->dev.bar, 0, kBarrierClear, st);
     if (e != cudaSuccess) return e;
     if (c->cg_strategy == B3G_CG_PERSISTENT_FUSED) return launch_grid_cg_fused(c->dev, dot, c->dev.bar, c->cg_rec, st);
     return launch_grid_cg(c->dev, dot, c->dev.bar, st);
+}
+
+// The status of a step that did not succeed.  A wait that gave up leaves the
+// barrier's counts short: the next solve starts from cleared ones.
+b3g_status step_failed(b3g_cloth* c, uint32_t status)
+{
+    if (status == (uint32_t)B3G_ERR_TIMEOUT) B3G_TRY(cudaMemsetAsync(c->dev.bar, 0, kBarrierReset, c->stream));
+    return (b3g_status)status;
 }
 
 // Captures one step: [contacts_update] assemble cg_init while{cg iteration}
@@ -348,6 +359,7 @@ b3g_status layout_cloth(b3g_cloth* c)
     d.nmouse = nmouse;
     d.nslices = T.nslices;
     d.max_deg = T.max_deg;
+    d.band = T.band;
     d.E = T.E;
     d.k_stretch = def->streching;
     d.k_shear = def->shearing;
@@ -372,7 +384,8 @@ b3g_status layout_cloth(b3g_cloth* c)
     add(nn); add(nn); add(nn * 4); add(nn * 12); add(nn * 12); add(nn * 12); add(nn * 12); add(nn * 12);
     add(sizeof(StepScalars));
     add(sizeof(GridBarrier));
-    add(std::max((size_t)d.grid * 32, kGridCgPartialBytes));
+    // (a server's cloths run no persistent CG of their own)
+    add(std::max((size_t)d.grid * 32, c->lean_layout ? kGridCgCounterBytes : kGridCgPartialBytes));
     add(vec); add(n);                       // staging
     add(T.E); add(n);                       // the assembly's first-touch order and its length
     if (T.slot_terms) {                     // slot-major assembly: term lists and element records
@@ -495,7 +508,7 @@ b3g_status realize_cloth(b3g_cloth* c, int device, char* base, bool owns_arena, 
     d.c_point = A.take<float>(3 * nn);
     d.sc = A.take<StepScalars>(1);
     d.bar = A.take<GridBarrier>(1);
-    d.partials = A.take<char>(std::max((size_t)d.grid * 32, kGridCgPartialBytes));
+    d.partials = A.take<char>(std::max((size_t)d.grid * 32, c->lean_layout ? kGridCgCounterBytes : kGridCgPartialBytes));
     c->d_stage = A.take<float>(3 * (size_t)n);
     c->d_stage_u8 = A.take<uint8_t>(n);
     d.asm_touch = A.take<uint8_t>(T.E);
@@ -1679,7 +1692,7 @@ b3g_status b3g_cloth_step(b3g_cloth* c, float dt, uint32_t vel_iters, uint32_t p
         count_launches(ns + hulls + 2 + cg + 1 + (ns && pos_iters > 1 ? pos_iters - 1 : 0) + 1);
     }
     if (stats) *stats = L;
-    if (dt > 0.0f && h->status != 0) return (b3g_status)h->status;
+    if (dt > 0.0f && h->status != 0) return step_failed(c, h->status);
     return B3G_OK;
 }
 
@@ -1780,7 +1793,7 @@ b3g_status b3g_cloth_step_profiled(b3g_cloth* c, float dt, uint32_t vel_iters, u
                 times->cg_update_ms + times->cg_direction_ms + times->finalize_ms + times->contact_position_ms +
                 times->post_ms;
     if (stats) *stats = L;
-    if (h->status != 0) return (b3g_status)h->status;
+    if (h->status != 0) return step_failed(c, h->status);
     return B3G_OK;
 }
 
@@ -1790,22 +1803,27 @@ b3g_status b3g_debug_cg_barrier_timeout(b3g_cloth* c, uint32_t spin_limit, b3g_s
     cudaSetDevice(c->device);
     cudaStream_t st = c->stream;
     // a barrier that cannot complete: the arrival counter starts half its
-    // range away from every target, so every CTA waits until its limit
-    GridBarrier bar = {0x80000000u, 0u, 0u, spin_limit};
+    // range away from every target (the on-chip CG publishes no partials when
+    // it is not zero), so every CTA waits until its limit
+    GridBarrier bar = {0x80000000u, 0u, spin_limit, 0u};
     StepScalars* h = c->h_sc;
     B3G_TRY(cudaStreamSynchronize(st));
     fill_step_scalars(c, 1.0f / 60.0f, 8, 2, h);
     c->step_index -= 1;
     B3G_TRY(cudaMemcpyAsync(c->dev.sc, h, sizeof(StepScalars), cudaMemcpyHostToDevice, st));
-    B3G_TRY(cudaMemcpyAsync(c->dev.bar, &bar, sizeof(bar), cudaMemcpyHostToDevice, st));
+    B3G_TRY(cudaMemcpyAsync(c->dev.bar, &bar, kBarrierClear, cudaMemcpyHostToDevice, st));
     B3G_TRY(launch_assemble(c->dev, c->assemble_block, st));
     if (c->cg_strategy == B3G_CG_PERSISTENT_FUSED) {
         b3g_status s = ensure_cg_rec(c);
         if (s != B3G_OK) return s;
         B3G_TRY(launch_grid_cg_fused(c->dev, (int)c->opts.dot, c->dev.bar, c->cg_rec, st));
     } else {
-        B3G_TRY(launch_grid_cg(c->dev, (int)c->opts.dot, c->dev.bar, st));
+        // (a cloth solved by one cluster waits on hardware barriers only)
+        const ResShape shape = resident_shape(c->dev);
+        B3G_TRY(shape.ctas && shape.grid ? launch_resident_cg(c->dev, shape, (int)c->opts.dot, st)
+                                         : launch_grid_cg(c->dev, (int)c->opts.dot, c->dev.bar, st));
     }
+    B3G_TRY(cudaMemsetAsync(c->dev.bar, 0, kBarrierReset, st));
     B3G_TRY(cudaMemcpyAsync(h, c->dev.sc, sizeof(StepScalars), cudaMemcpyDeviceToHost, st));
     B3G_TRY(cudaStreamSynchronize(st));
     *result = (b3g_status)h->status;

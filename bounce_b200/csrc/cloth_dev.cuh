@@ -88,6 +88,7 @@ void rank_colliders(SphereDev* sph, uint32_t count);
 struct ClothDev {
     uint32_t n, t, ns, nsph;
     uint32_t nslices, max_deg, E;
+    uint32_t band;              // widest |row - column| of the matrix
     const uint32_t* slice_off;  // nslices + 1
     const uint8_t* row_deg;     // n
     const uint32_t* cols;       // E

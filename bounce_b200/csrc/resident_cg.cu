@@ -1,0 +1,150 @@
+// Launches of the on-chip MPCG (resident_cg.cuh) for one cloth.
+#include "resident_cg.h"
+
+#include <algorithm>
+
+#include "resident_cg.cuh"
+
+namespace b3g {
+
+namespace {
+
+template <int DOT, int RPT>
+__global__ void __launch_bounds__(kResMaxThreads, 1)
+    k_resident_team(const __grid_constant__ ClothDev c, uint32_t chunk, uint32_t wide, uint32_t smem_bytes)
+{
+    extern __shared__ __align__(128) char smem[];
+    ResShared* sh = reinterpret_cast<ResShared*>(smem);
+    TeamScope team;
+    team.size = gridDim.x;  // one cluster
+    team.rank = blockIdx.x;
+    team.parity = 0u;
+    team.sh = sh;
+    team.zs = reinterpret_cast<float*>(smem + kResHeader) + 3u * (size_t)res_window(c.n, chunk, c.band);
+    uint32_t phase = 0u;
+    res_init_copy_barrier(sh);
+    resident_solve<DOT, RPT>(c, team, smem, chunk, wide != 0u, smem_bytes, phase);
+    team.barrier();  // no CTA leaves while another may still write into it
+}
+
+template <int DOT, int RPT>
+__global__ void __launch_bounds__(kResMaxThreads, 1)
+    k_resident_grid(const __grid_constant__ ClothDev c, uint32_t chunk, uint32_t wide, uint32_t smem_bytes)
+{
+    extern __shared__ __align__(128) char smem[];
+    ResShared* sh = reinterpret_cast<ResShared*>(smem);
+    GridScope team;
+    team.size = gridDim.x;
+    team.rank = blockIdx.x;
+    team.epoch = 0u;
+    team.sh = sh;
+    team.bar = c.bar;
+    team.part = reinterpret_cast<ulonglong2*>(static_cast<char*>(c.partials) + kGridCgCounterBytes);
+    team.base = *(volatile uint32_t*)&c.bar->nonce;
+    team.mute = *(volatile uint32_t*)&c.bar->count != 0u;
+    team.limit = c.bar->spin_limit ? c.bar->spin_limit : kResSpinLimit;
+    team.zt = reinterpret_cast<float4*>(c.p);  // p and s, 6 n floats, are free here
+    team.arrivals = *(volatile uint32_t*)&c.bar->arrivals;
+    uint32_t phase = 0u;
+    res_init_copy_barrier(sh);
+    const bool good = resident_solve<DOT, RPT>(c, team, smem, chunk, wide != 0u, smem_bytes, phase);
+    if (threadIdx.x == 0 && !good) {
+        c.sc->status = kResTimeout;
+        c.sc->cont = 0;
+    }
+    // the next launch's tags differ from this one's (a CTA that gave up may
+    // be a reduction behind the others)
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *(volatile uint32_t*)&c.bar->arrivals = team.arrivals + team.epoch * team.size;
+        *(volatile uint32_t*)&c.bar->nonce = team.base + team.epoch + 8u;
+    }
+}
+
+template <int DOT>
+const void* kernel_for(bool grid, uint32_t rpt)
+{
+    if (grid)
+        return rpt == 1 ? (const void*)k_resident_grid<DOT, 1> : (const void*)k_resident_grid<DOT, 2>;
+    return rpt == 1 ? (const void*)k_resident_team<DOT, 1> : (const void*)k_resident_team<DOT, 2>;
+}
+
+}  // namespace
+
+ResShape resident_shape(const ClothDev& c)
+{
+    ResShape s;
+    if (c.max_deg > (uint32_t)kResSlots || c.n == 0) return s;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const uint32_t n = c.n, slices = (n + 31u) / 32u;
+    auto shape = [&](bool grid, uint32_t ctas) {
+        ResShape r;
+        const uint32_t per = (slices + ctas - 1u) / ctas;
+        r.grid = grid;
+        r.chunk = 32u * per;
+        r.ctas = grid ? (n + r.chunk - 1u) / r.chunk : ctas;
+        r.rows_per_thread = r.chunk <= (uint32_t)kResMaxThreads ? 1u : 2u;
+        r.threads = 32u * ((per + r.rows_per_thread - 1u) / r.rows_per_thread);
+        // threads without rows of their own help with the halo
+        const uint32_t halo = std::min(n, r.chunk + 2u * c.band) - std::min(n, r.chunk);
+        const uint32_t most = grid || ctas == 1u ? (uint32_t)kResMaxThreads : 32u * kResTeamWarps;
+        r.threads = std::max(r.threads, std::min(most, 32u * ((halo + 32u * kResHalo - 1u) / (32u * kResHalo))));
+        if (grid) r.threads = std::max(r.threads, 32u * ((r.ctas + 31u) / 32u));  // a thread a partial
+        r.wide = halo > (uint32_t)kResHalo * r.threads;
+        const uint64_t off = res_block_offset(n, r.chunk, c.band, !grid && ctas > 1u, r.wide);
+        const uint64_t all = off + (uint64_t)r.chunk * c.max_deg * 36u;
+        r.smem = (uint32_t)std::min<uint64_t>(all, kResSmemLimit);
+        // at least half of the blocks resident
+        if (r.threads > most || off + (uint64_t)r.chunk * c.max_deg * 18u > kResSmemLimit) r.ctas = 0;
+        return r;
+    };
+    // One CTA to 256 rows, then clusters of up to 8 CTAs of 128 to 512 rows,
+    // then the grid.  Measured per iteration (FP64 dots, 7 blocks a row): 256
+    // rows 2.6 us on one CTA and 2.9 on two; 1,024 rows 3.3 on eight CTAs, 4.2
+    // on two; 4,096 rows 4.5 on eight and 6.2 on the grid; 8,281 rows (13
+    // blocks) 8.5 on a cluster of 16 and 5.4 on the grid.
+    uint32_t t = 1;
+    while (n > 256u && t < 8u && n > t * 128u) t *= 2;
+    if (n <= 8u * (uint32_t)kResMaxThreads) {
+        s = shape(false, t);
+        if (s.ctas) return s;
+    }
+    return shape(true, (uint32_t)std::min(sms, kResMaxGrid));
+}
+
+cudaError_t launch_resident_cg(const ClothDev& c, const ResShape& s, int dot, cudaStream_t st)
+{
+    const void* fn = dot == 2 ? kernel_for<2>(s.grid, s.rows_per_thread)
+                   : dot == 1 ? kernel_for<1>(s.grid, s.rows_per_thread) : kernel_for<0>(s.grid, s.rows_per_thread);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemLimit);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(s.ctas);
+    cfg.blockDim = dim3(s.threads);
+    cfg.dynamicSmemBytes = s.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (s.grid) {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    } else {
+        if (s.ctas > 8) {
+            e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (e != cudaSuccess) return e;
+        }
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = s.ctas;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    uint32_t chunk = s.chunk, wide = s.wide ? 1u : 0u, bytes = s.smem;
+    void* args[4] = {const_cast<ClothDev*>(&c), &chunk, &wide, &bytes};
+    e = cudaLaunchKernelExC(&cfg, fn, args);
+    count_launches(1);
+    return e;
+}
+
+}  // namespace b3g

@@ -1,0 +1,689 @@
+// The MPCG of one cloth with its system held on chip: device code shared by
+// the single-cloth launches (resident_cg.cu) and the batch (batch_cg.cu).
+//
+// A team of CTAs owns the cloth's rows in contiguous chunks, at most RPT rows
+// a thread.  For the whole solve a CTA keeps in shared memory
+//  * its rows' blocks, copied once by bulk copies in the SELL layout (a slice's
+//    component q is one contiguous run of 128 bytes a slot), as many slices as
+//    fit; the rest are read from L2 in every product;
+//  * the direction p of its window: its own rows and every row within `band`
+//    of them (band = the widest |row - column| of the matrix), so a product
+//    gathers p from shared memory only.
+// x, r, z, p and P^-1 of its own rows and their column indices stay in
+// registers.  Per iteration only z of the window's halo crosses CTAs: the
+// halo's p = z + beta p_old is formed where it is needed, from the same float
+// expression as its owner's.
+//
+// An iteration (b3SolveMPCG, src/bounce/cloth/cloth_force_solver.cpp:61-136):
+//   A: p = z + beta p_old, s = S A p, p.s                     -> alpha
+//   B: x += alpha p, r -= alpha s, z = S P^-1 r, r.z          -> delta', beta
+// Each phase ends in a team reduction; B's also publishes z.
+//
+// Two kinds of team:
+//  * TeamScope: one CTA, or a cluster whose CTAs store their partials into
+//    each other's shared memory; one cluster barrier a reduction, z read from
+//    the owner's shared memory.
+//  * GridScope: the CTAs of a cooperative launch.  Partials and rows of z are
+//    published as 16-byte words that carry a tag of the launch and the
+//    reduction, so that a reader knows whether it has them: no fence (one a
+//    phase costs 0.75 us), only a count of arrivals.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "cg_common.cuh"
+#include "cloth_dev.cuh"
+#include "grid_cg.cuh"
+#include "resident_cg.h"
+#include "vec.cuh"
+
+namespace b3g {
+
+namespace {
+
+namespace rcg = cooperative_groups;
+
+constexpr int kResMaxWarps = kResMaxThreads / 32;
+constexpr uint32_t kResSpinLimit = 1u << 24;
+constexpr uint32_t kResTimeout = 7;  // B3G_ERR_TIMEOUT
+
+// The fixed part of the shared memory.
+struct ResShared {
+    double wsum[2][2][kResMaxTeam * kResTeamWarps];  // [parity][value][rank and warp]
+    unsigned long long mbar;
+    int lost;
+    uint32_t listed;  // wide windows: halo rows the CTA's rows touch
+};
+static_assert(sizeof(ResShared) <= kResHeader, "fixed shared memory of the resident CG");
+static_assert(kResMaxWarps <= kResMaxTeam * kResTeamWarps, "a CTA alone keeps every warp's sum");
+
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// ---- sums -------------------------------------------------------------------
+
+template <class T>
+__device__ __forceinline__ unsigned long long pack8(T a)
+{
+    unsigned long long u = 0ull;
+    memcpy(&u, &a, sizeof(T));
+    return u;
+}
+template <class T>
+__device__ __forceinline__ T unpack8(unsigned long long u)
+{
+    T a;
+    memcpy(&a, &u, sizeof(T));
+    return a;
+}
+
+template <class D>
+__device__ __forceinline__ typename D::T warp_sum(typename D::T v)
+{
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v = D::combine(v, D::shfl(v, off));
+    return v;
+}
+
+// The sum of `count` 8-byte words in shared memory, in a fixed tree, by one
+// thread: no shuffles.
+template <class D>
+__device__ __forceinline__ typename D::T words_sum(const double* w, uint32_t count)
+{
+    typedef typename D::T T;
+    T a[kResMaxWarps];
+#pragma unroll
+    for (uint32_t k = 0; k < (uint32_t)kResMaxWarps; ++k)
+        a[k] = k < count ? *reinterpret_cast<const T*>(w + k) : D::zero();
+#pragma unroll
+    for (int step = kResMaxWarps / 2; step > 0; step >>= 1)
+#pragma unroll
+        for (int k = 0; k < step; ++k) a[k] = D::combine(a[k], a[k + step]);
+    return a[0];
+}
+
+// One CTA (size 1) or the CTAs of a thread-block cluster.
+struct TeamScope {
+    static constexpr bool kGrid = false;
+    uint32_t rank, size, parity;
+    ResShared* sh;
+    float* zs;  // 3 planes of `chunk`: z of this CTA's rows, read by the team
+
+    __device__ void barrier() const
+    {
+        if (size == 1) __syncthreads();
+        else rcg::this_cluster().sync();
+    }
+
+    // The team's sums, the same in every thread: every warp stores its sum
+    // into each CTA of the team, one barrier, and every thread adds them up.
+    // A buffer is written again only two reductions later, after the barrier
+    // in between.
+    template <class D, int NV>
+    __device__ bool sum(typename D::T (&v)[NV])
+    {
+        typedef typename D::T T;
+        const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        parity ^= 1u;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const unsigned long long u = __shfl_sync(0xffffffffu, pack8(warp_sum<D>(v[k])), 0);
+            double* mine = &sh->wsum[parity][k][rank * nw + warp];
+            if (lane < size) {
+                double* to = size == 1 ? mine : rcg::this_cluster().map_shared_rank(mine, lane);
+                *reinterpret_cast<unsigned long long*>(to) = u;
+            }
+        }
+        barrier();
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const double* w = sh->wsum[parity][k];
+            if (size * nw <= (uint32_t)kResMaxWarps) {
+                v[k] = words_sum<D>(w, size * nw);
+            } else {
+                T a = D::zero();
+                for (uint32_t i = lane; i < size * nw; i += 32u) a = D::combine(a, *reinterpret_cast<const T*>(w + i));
+                v[k] = unpack8<T>(__shfl_sync(0xffffffffu, pack8(warp_sum<D>(a)), 0));
+            }
+        }
+        return true;
+    }
+    __device__ void put_z(const ClothDev&, uint32_t, uint32_t local, uint32_t chunk, f3 z) const
+    {
+        if (size > 1) st3(zs, chunk, local, z);
+    }
+    __device__ f3 get_z(const ClothDev&, uint32_t row, uint32_t chunk, uint32_t) const
+    {
+        const uint32_t owner = row / chunk;
+        return ld3(rcg::this_cluster().map_shared_rank(zs, owner), chunk, row - owner * chunk);
+    }
+};
+
+// The CTAs of a cooperative launch.
+struct GridScope {
+    static constexpr bool kGrid = true;
+    uint32_t rank, size, epoch, base, arrivals;
+    ResShared* sh;
+    GridBarrier* bar;
+    ulonglong2* part;  // [parity][value][rank], a line each
+    float4* zt;        // z of every row and a tag of the reduction that follows it
+    uint32_t limit;
+    bool mute;         // the diagnostic of the bounded waits: nothing is published
+
+    static __device__ void put(ulonglong2* p, unsigned long long v, unsigned long long tag)
+    {
+        asm volatile("{.reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t;}" ::"l"(p), "l"(v),
+                     "l"(tag)
+                     : "memory");
+    }
+    static __device__ void get(const ulonglong2* p, unsigned long long& v, unsigned long long& tag)
+    {
+        asm volatile("{.reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t;}"
+                     : "=l"(v), "=l"(tag)
+                     : "l"(p)
+                     : "memory");
+    }
+    __device__ bool failed() const { return *(volatile uint32_t*)&bar->error == base + 1u; }
+    __device__ void fail() const { *(volatile uint32_t*)&bar->error = base + 1u; }
+
+    // A row's z travels with its tag in one 16-byte word, so whoever reads
+    // the tag has the row: no fence, and the reduction that follows moves no
+    // data but its partials.  The tag is a NaN that no arithmetic makes.
+    __device__ uint32_t z_tag() const { return 0xffc00000u | ((base + epoch) & 0x3fffffu); }
+    __device__ void put_z(const ClothDev&, uint32_t row, uint32_t, uint32_t, f3 z) const
+    {
+        if (mute) return;
+        put(reinterpret_cast<ulonglong2*>(zt + row),
+            (unsigned long long)__float_as_uint(z.x) | ((unsigned long long)__float_as_uint(z.y) << 32),
+            (unsigned long long)__float_as_uint(z.z) | ((unsigned long long)z_tag() << 32));
+    }
+    // Row `row` as published under `tag`; the wait is bounded.
+    __device__ f3 get_z(const ClothDev&, uint32_t row, uint32_t, uint32_t tag) const
+    {
+        unsigned long long a, b;
+        for (uint32_t spins = 0;; ++spins) {
+            get(reinterpret_cast<const ulonglong2*>(zt + row), a, b);
+            if ((uint32_t)(b >> 32) == tag) break;
+            if (spins > limit || ((spins & 63u) == 63u && failed())) {
+                sh->lost = 1;
+                fail();
+                break;
+            }
+        }
+        return f3{__uint_as_float((uint32_t)a), __uint_as_float((uint32_t)(a >> 32)), __uint_as_float((uint32_t)b)};
+    }
+
+    // The grid's sums.  Each CTA counts itself in and publishes its partial as
+    // one tagged 16-byte word in a line of its own; once the count is full,
+    // thread r of every CTA reads rank r's partial, and all sum them in the
+    // same order (a shuffle tree a warp, then the warps in order).  Neither the
+    // count nor the partials carry a fence: a partial that is not there yet is
+    // known by its tag and looked at again.  One thread a CTA polls the count
+    // because polling all partials from every CTA delays the stores they wait
+    // for (an all-reduce of 148 CTAs: 1.2 us polling the count, 3.5 us and more
+    // polling the partials while CTAs arrive apart, or with several partials a
+    // line).  Two buffers suffice: a CTA publishes reduction e + 2 only once
+    // every CTA has counted itself in for e + 1, and so has read e.  The waits
+    // are bounded; false (in every thread) on error.
+    template <class D, int NV>
+    __device__ void publish(typename D::T (&v)[NV])
+    {
+        typedef typename D::T T;
+        const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        ++epoch;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const T a = warp_sum<D>(v[k]);
+            if (lane == 0) *reinterpret_cast<T*>(&sh->wsum[0][k][warp]) = a;
+        }
+        __syncthreads();
+        if (mute) return;
+        if (threadIdx.x == 0)
+            asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(&bar->arrived) : "memory");
+        if (threadIdx.x < (uint32_t)NV)
+            put(part + (((epoch & 1u) * 2u + lane) * kResMaxGrid + rank) * kResLine,
+                pack8(words_sum<D>(sh->wsum[0][lane], nw)), base + epoch);
+    }
+    template <class D, int NV>
+    __device__ bool collect(typename D::T (&v)[NV])
+    {
+        typedef typename D::T T;
+        const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+        if (threadIdx.x == 0) {
+            const uint32_t target = arrivals + epoch * size;
+            for (uint32_t spins = 0;; ++spins) {
+                uint32_t a;
+                asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(a) : "l"(&bar->arrived) : "memory");
+                if ((int32_t)(a - target) >= 0) break;
+                if (spins > limit || ((spins & 63u) == 63u && failed())) {
+                    sh->lost = 1;
+                    fail();
+                    break;
+                }
+            }
+        }
+        __syncthreads();
+        if (warp * 32u < size) {
+            const ulonglong2* buf = part + ((epoch & 1u) * 2u * kResMaxGrid + threadIdx.x) * kResLine;
+            const unsigned long long tag = base + epoch;
+            const bool mine = threadIdx.x < size;
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                T a = D::zero();
+                if (mine) {
+                    unsigned long long u, t;
+                    for (uint32_t spins = 0;; ++spins) {
+                        get(buf + k * kResMaxGrid * kResLine, u, t);
+                        if (t == tag) break;
+                        if (spins > limit || ((spins & 63u) == 63u && failed())) {
+                            sh->lost = 1;
+                            fail();
+                            break;
+                        }
+                    }
+                    a = unpack8<T>(u);
+                }
+                a = warp_sum<D>(a);
+                if (lane == 0) *reinterpret_cast<T*>(&sh->wsum[1][k][warp]) = a;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            T a = *reinterpret_cast<const T*>(&sh->wsum[1][k][0]);
+#pragma unroll
+            for (uint32_t w = 1; w < (uint32_t)kResMaxGrid / 32u; ++w)
+                if (32u * w < size) a = D::combine(a, *reinterpret_cast<const T*>(&sh->wsum[1][k][w]));
+            v[k] = a;
+        }
+        return sh->lost == 0;
+    }
+};
+
+// ---- the solve --------------------------------------------------------------
+
+// cg_stop (cg_common.cuh) with its bound computed once.
+struct StopBound {
+    double bound = 0.0;
+    bool single = false;
+    __device__ StopBound() {}
+    __device__ StopBound(const StepScalars* sc, double b_delta, int dot)
+    {
+        const double tol = (double)sc->tol;
+        single = sc->stop_rule == 0 && dot != 2;
+        bound = sc->stop_rule != 0 ? tol * tol * b_delta
+                : single           ? (double)(kEps * kEps * (float)b_delta)
+                                   : (double)(kEps * kEps) * b_delta;
+    }
+    __device__ bool met(double delta) const { return (single ? (double)(float)delta : delta) <= bound; }
+};
+
+// One row: its blocks' first word (in the resident blocks or in ClothDev::vals),
+// the distance of their components, its slice's width, and the window indices
+// of its columns, two a word.
+struct ResRow {
+    uint32_t off, cs, width;
+    uint32_t col[kResSlots / 2];
+};
+
+template <int I>
+struct ResInt {
+    static constexpr int value = I;
+};
+
+// Word `q` cs of slot K: in shared memory at byte address a (+ 128 K), or in global memory.
+template <int K>
+__device__ __forceinline__ float res_word(uint32_t a)
+{
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1+%2];" : "=f"(v) : "r"(a), "n"(128 * K));
+    return v;
+}
+template <int K>
+__device__ __forceinline__ float res_word(const float* a)
+{
+    return a[32 * K];
+}
+
+// p of window row j: three words a row, so that a warp's rows fall on
+// different banks and one address serves the three.
+__device__ __forceinline__ f3 ldp(const float* P, uint32_t j) { return f3{P[3 * j], P[3 * j + 1], P[3 * j + 2]}; }
+__device__ __forceinline__ void stp(float* P, uint32_t j, f3 v)
+{
+    P[3 * j] = v.x;
+    P[3 * j + 1] = v.y;
+    P[3 * j + 2] = v.z;
+}
+
+// The blocks and directions of slots K .. K + G - 1, then their products in
+// slot order, acc = acc + A_k p_k (b3Mat33 * b3Vec3, include/bounce/common/
+// math/mat33.h:129-132): the loads of the G slots are in flight together.
+template <int K, int G, class A>
+__device__ __forceinline__ f3 res_slots(f3 acc, const ResRow& r, const A (&a)[9], const float* P)
+{
+    m3 m[G];
+    f3 p[G];
+    auto load = [&](auto g) {
+        constexpr int k = K + decltype(g)::value;
+        p[k - K] = ldp(P, (k & 1) ? r.col[k >> 1] >> 16 : r.col[k >> 1] & 0xffffu);
+        m[k - K] = m3{f3{res_word<k>(a[0]), res_word<k>(a[1]), res_word<k>(a[2])},
+                      f3{res_word<k>(a[3]), res_word<k>(a[4]), res_word<k>(a[5])},
+                      f3{res_word<k>(a[6]), res_word<k>(a[7]), res_word<k>(a[8])}};
+    };
+    load(ResInt<0>());
+    if constexpr (G > 1) load(ResInt<1>());
+    if constexpr (G > 2) load(ResInt<2>()), load(ResInt<3>());
+#pragma unroll
+    for (int g = 0; g < G; ++g) acc = acc + m[g] * p[g];
+    return acc;
+}
+
+// s_i = sum_k A_k p_k of one row.  The warp walks its slice's width (a row's
+// padding holds zero blocks on the diagonal's column): fours, then a pair and
+// a single slot.
+template <int K, class A>
+__device__ __forceinline__ f3 res_walk(f3 acc, const ResRow& r, const A (&a)[9], const float* P)
+{
+    if constexpr (K < kResSlots) {
+        if (K + 4u <= r.width) {
+            acc = res_slots<K, 4>(acc, r, a, P);
+            return res_walk<K + 4>(acc, r, a, P);
+        }
+        if (K + 2u <= r.width) {
+            acc = res_slots<K, 2>(acc, r, a, P);
+            if (K + 3u == r.width) acc = res_slots<K + 2, 1>(acc, r, a, P);
+        } else if (K + 1u == r.width) {
+            acc = res_slots<K, 1>(acc, r, a, P);
+        }
+    }
+    return acc;
+}
+__device__ __forceinline__ f3 res_row_times(const ResRow& r, uint32_t blocks, const float* P)
+{
+    uint32_t a[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) a[q] = blocks + 4u * (r.off + q * r.cs);
+    return res_walk<0>(zero3(), r, a, P);
+}
+__device__ __forceinline__ f3 res_row_times(const ResRow& r, const float* blocks, const float* P)
+{
+    const float* a[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) a[q] = blocks + r.off + (size_t)q * r.cs;
+    return res_walk<0>(zero3(), r, a, P);
+}
+
+// The whole solve by a team.  `smem`: kResHeader bytes (the scope's
+// ResShared), then P (3 W floats), zs (3 chunk floats, clusters only), then
+// the blocks from a_off on, up to smem_bytes.  `wide`: most of the window is
+// not needed (few couplings reach far), so the CTA lists the halo rows that
+// its rows touch.  `phase`: the copy barrier's
+// phase, kept over the solves of a persistent launch; the barrier is
+// initialised by the caller.  Returns false when a bounded wait gave up.
+template <int DOT, int RPT, class S>
+__device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t chunk, bool wide,
+                               uint32_t smem_bytes, uint32_t& phase)
+{
+    typedef DotT<DOT> D;
+    typedef typename D::T T;
+    const uint32_t n = c.n, B = blockDim.x, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nw = B >> 5;
+    const StepScalars* sc = c.sc;
+    const uint32_t r0 = min(n, team.rank * chunk), r1 = min(n, r0 + chunk);
+    const bool empty = r0 == r1;  // a CTA past the last row still joins the reductions
+    const uint32_t w0 = empty ? r0 : r0 > c.band ? r0 - c.band : 0u, w1 = empty ? r0 : min(n, r1 + c.band);
+    const uint32_t W = res_window(n, chunk, c.band);
+    float* P = reinterpret_cast<float*>(smem + kResHeader);
+    const bool zin = !S::kGrid && team.size > 1;
+    const uint32_t a_off = res_block_offset(n, chunk, c.band, zin, wide);
+    uint16_t* list = reinterpret_cast<uint16_t*>(smem + kResHeader + 12u * W + (zin ? 12u * chunk : 0u));
+    uint8_t* seen = reinterpret_cast<uint8_t*>(list + W);
+    float* As = reinterpret_cast<float*>(smem + a_off);
+    const uint32_t q0 = r0 >> 5, q1 = empty ? q0 : (r1 + 31u) >> 5;
+    const uint32_t so0 = c.slice_off[q0];
+    const uint32_t room = (smem_bytes - a_off) / 36u;  // blocks
+
+    // the resident slices: the first ones that fit
+    uint32_t qr = q1;
+    while (qr > q0 && c.slice_off[qr] - so0 > room) --qr;
+    const bool copies = qr > q0;
+    if (copies) {
+        __syncthreads();  // an earlier solve's reads of the buffer are done
+        if (tid == 0) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&team.sh->mbar)),
+                         "r"((c.slice_off[qr] - so0) * 36u)
+                         : "memory");
+        }
+        __syncthreads();
+        for (uint32_t k = tid; k < 9u * (qr - q0); k += B) {
+            const uint32_t q = q0 + k / 9u, comp = k % 9u;
+            const uint32_t so = c.slice_off[q], len = c.slice_off[q + 1] - so;
+            if (len)
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                        smem_addr(As + 9u * (size_t)(so - so0) + (size_t)comp * len)),
+                    "l"(c.vals + (size_t)comp * c.E + so), "r"(len * 4u), "r"(smem_addr(&team.sh->mbar))
+                    : "memory");
+        }
+    }
+
+    ResRow row[RPT];
+    f3 x[RPT], r[RPT], z[RPT], p[RPT], pv[RPT], s[RPT];
+    uint32_t flags = 0u;  // per row: bit i active, bit 8 + i dynamic, bit 16 + i resident
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+        const uint32_t q = q0 + warp + i * nw, g = 32u * q + lane;
+        row[i].off = row[i].cs = row[i].width = 0u;
+        x[i] = r[i] = z[i] = p[i] = s[i] = pv[i] = zero3();
+#pragma unroll
+        for (int k = 0; k < kResSlots / 2; ++k) row[i].col[k] = 0u;
+        if (q < q1 && g < r1) {
+            const uint32_t so = c.slice_off[q];
+            const bool res = q < qr;
+            const bool dyn = c.type[g] == 2;
+            flags |= (1u << i) | (dyn ? 0x100u << i : 0u) | (res ? 0x10000u << i : 0u);
+            const uint32_t len = c.slice_off[q + 1] - so;
+            row[i].width = len >> 5;
+            row[i].cs = res ? len : c.E;
+            row[i].off = (res ? 9u * (so - so0) : so) + lane;
+#pragma unroll
+            for (int k = 0; k < kResSlots; ++k)
+                if ((uint32_t)k < row[i].width) row[i].col[k >> 1] |= (c.cols[so + lane + 32u * k] - w0) << ((k & 1) * 16);
+            pv[i] = ld3(c.pinv, n, g);
+        }
+    }
+    const uint32_t below = r0 - w0;
+    uint32_t halo = below + (w1 - r1);
+    if (wide) {
+        for (uint32_t l = tid; l < W; l += B) seen[l] = 0;
+        if (tid == 0) team.sh->listed = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+#pragma unroll
+            for (int k = 0; k < kResSlots; ++k)
+                if ((uint32_t)k < row[i].width) seen[(k & 1) ? row[i].col[k >> 1] >> 16 : row[i].col[k >> 1] & 0xffffu] = 1;
+        __syncthreads();
+        for (uint32_t l = tid; l < w1 - w0; l += B)
+            if (seen[l] && (l < below || l >= r1 - w0)) list[atomicAdd(&team.sh->listed, 1u)] = (uint16_t)l;
+        __syncthreads();
+        halo = team.sh->listed;
+    }
+    // the window index of halo row h
+    auto halo_at = [&](uint32_t h) -> uint32_t { return wide ? list[h] : h < below ? h : r1 - w0 + (h - below); };
+    // x0 = S m_x over the window (cg_soft: on every row)
+    for (uint32_t j = w0 + tid; j < w1; j += B)
+        stp(P, j - w0, (c.cg_soft || c.type[j] == 2) ? ld3(c.mx, n, j) : zero3());
+    bool landed = true;
+    if (copies) {
+        const uint32_t mb = smem_addr(&team.sh->mbar);
+        uint32_t done = 0u;
+        for (uint32_t t = 0; !done && t < (1u << 20); ++t)
+            asm volatile("{.reg .pred q; mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2; selp.u32 %0, 1, 0, q;}"
+                         : "=r"(done)
+                         : "r"(mb), "r"(phase)
+                         : "memory");
+        phase ^= 1u;
+        landed = done != 0u;
+    }
+    __syncthreads();
+
+    const uint32_t as_addr = smem_addr(As);
+    f3 zh[kResHalo];  // z of the thread's first halo rows
+    uint32_t tag = 0u;
+    // the sums of the phase that made z, and the halo's z
+    auto sum_and_halo = [&](auto& v) -> bool {
+        constexpr int NV = sizeof(v) / sizeof(v[0]);
+        bool good;
+        if constexpr (S::kGrid) {
+            tag = team.z_tag();
+            team.template publish<D, NV>(v);
+            good = team.template collect<D, NV>(v);
+        } else {
+            good = team.template sum<D, NV>(v);
+        }
+#pragma unroll
+        for (int u = 0; u < kResHalo; ++u) {
+            const uint32_t h = tid + u * B;
+            if (h < halo) zh[u] = team.get_z(c, w0 + halo_at(h), chunk, tag);
+        }
+        return good;
+    };
+    const uint32_t max_iter = sc->max_iter;
+    uint32_t it = 0, status = 0u;
+    float beta = 0.0f;
+    double b_delta = 0.0, delta = 0.0, delta0 = 0.0;
+    StopBound stop;
+    // The first pass multiplies A x0, every later one A p.
+    for (bool start = true;; start = false) {
+        if (!start) {
+            // the window's p = z + beta p_old (cloth_force_solver.cpp:130)
+            const bool first = it == 0;
+#pragma unroll
+            for (int u = 0; u < kResHalo; ++u) {
+                const uint32_t h = tid + u * B;
+                if (h < halo) {
+                    const uint32_t l = halo_at(h);
+                    stp(P, l, first ? zh[u] : zh[u] + beta * ldp(P, l));
+                }
+            }
+            for (uint32_t h = tid + kResHalo * B; h < halo; h += B) {
+                const uint32_t l = halo_at(h);
+                const f3 zj = team.get_z(c, w0 + l, chunk, tag);
+                stp(P, l, first ? zj : zj + beta * ldp(P, l));
+            }
+#pragma unroll
+            for (int i = 0; i < RPT; ++i)
+                if ((flags >> i) & 1u) {
+                    p[i] = first ? z[i] : z[i] + beta * p[i];
+                    stp(P, below + 32u * (warp + i * nw) + lane, p[i]);
+                }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            s[i] = zero3();
+            if ((flags >> (16 + i)) & 1u) s[i] = res_row_times(row[i], as_addr, P);
+            else if (row[i].width) s[i] = res_row_times(row[i], c.vals, P);
+            if (!((flags >> (8 + i)) & 1u) && !start) s[i] = zero3();
+        }
+        if (start) {
+            // r = S (b - A x0), z = S P^-1 r, b_delta, delta (cloth_force_solver.cpp:90-100;
+            // softbody_force_solver.cpp:93-127 with cg_soft)
+            T v2[2] = {D::zero(), D::zero()};
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) {
+                if ((flags >> i) & 1u) {
+                    const uint32_t l = 32u * (warp + i * nw) + lane, g = r0 + l;
+                    const bool dyn = (flags >> (8 + i)) & 1u;
+                    const f3 bi = ld3(c.b, n, g);
+                    x[i] = ldp(P, g - w0);
+                    r[i] = dyn ? bi - s[i] : zero3();
+                    z[i] = dyn ? mk(r[i].x * pv[i].x, r[i].y * pv[i].y, r[i].z * pv[i].z) : zero3();
+                    team.put_z(c, g, l, chunk, z[i]);
+                    const f3 bh = dyn ? bi : zero3();
+                    const f3 w = c.cg_soft ? ld3(c.cg_diag, n, g) : pv[i];
+                    v2[0] = D::add_term(v2[0], bh, mk(bh.x * w.x, bh.y * w.y, bh.z * w.z));
+                    v2[1] = D::add_term(v2[1], r[i], z[i]);
+                }
+            }
+            // a copy that never landed ends the whole team's solve as a breakdown
+            if (!landed) v2[1] = D::add_term(v2[1], mk(NAN, NAN, NAN), mk(1.0f, 1.0f, 1.0f));
+            __syncthreads();  // P is written again below
+            if (!sum_and_halo(v2)) return false;
+            b_delta = D::value(v2[0]), delta = D::value(v2[1]);
+            if (DOT != 2) {
+                b_delta = (double)(float)b_delta;
+                delta = (double)(float)delta;
+            }
+            delta0 = delta;
+            if (!isfinite(delta) || !isfinite(b_delta)) status = kStatusNumerical;
+            stop = StopBound(sc, b_delta, DOT);
+            if (status != 0u || max_iter == 0u || stop.met(delta)) break;
+            continue;
+        }
+        // alpha = delta / p.s (cloth_force_solver.cpp:115-117)
+        T v1[1] = {D::zero()};
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+            if ((flags >> i) & 1u) v1[0] = D::add_term(v1[0], p[i], s[i]);
+        if constexpr (S::kGrid) {
+            team.template publish<D, 1>(v1);
+            if (!team.template collect<D, 1>(v1)) return false;
+        } else {
+            team.template sum<D, 1>(v1);
+        }
+        const double pAp = D::value(v1[0]);
+        const float alpha = DOT == 2 ? (float)(delta / pAp) : (float)delta / (float)pAp;
+        // the update (cloth_force_solver.cpp:119-128)
+        T u1[1] = {D::zero()};
+#pragma unroll
+        for (int i = 0; i < RPT; ++i)
+            if ((flags >> i) & 1u) {
+                const uint32_t l = 32u * (warp + i * nw) + lane;
+                x[i] = x[i] + alpha * p[i];
+                r[i] = r[i] - alpha * s[i];
+                const f3 h = mk(r[i].x * pv[i].x, r[i].y * pv[i].y, r[i].z * pv[i].z);
+                z[i] = (flags >> (8 + i)) & 1u ? h : zero3();
+                team.put_z(c, r0 + l, l, chunk, z[i]);
+                u1[0] = D::add_term(u1[0], r[i], h);
+            }
+        if (!sum_and_halo(u1)) return false;
+        double dn = D::value(u1[0]);
+        if (DOT == 2) {
+            beta = (float)(dn / delta);
+        } else {
+            dn = (double)(float)dn;
+            beta = (float)dn / (float)delta;
+        }
+        delta = dn;
+        ++it;
+        if (!isfinite(dn) || !isfinite(alpha) || !isfinite(beta)) status = kStatusNumerical;
+        if (status != 0u || it >= max_iter || stop.met(dn)) break;
+    }
+#pragma unroll
+    for (int i = 0; i < RPT; ++i)
+        if ((flags >> i) & 1u) st3(c.dv, n, r0 + 32u * (warp + i * nw) + lane, x[i]);
+    if (team.rank == 0 && tid == 0) {
+        StepScalars* w = c.sc;
+        w->b_delta = b_delta;
+        w->delta0 = delta0;
+        w->delta = delta;
+        w->iter = it;
+        w->status = status;
+        w->cont = 0;
+    }
+    return true;
+}
+
+__device__ __forceinline__ void res_init_copy_barrier(ResShared* sh)
+{
+    if (threadIdx.x == 0) {
+        sh->lost = 0;
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sh->mbar)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+}
+
+}  // namespace
+}  // namespace b3g

@@ -865,7 +865,7 @@ b3g_status persistent_cg(b3g_softbody* b, cudaStream_t s, StepScalars* h)
     init.tol = b->opts.tolerance;
     init.dot = (int)b->opts.dot;
     SB_TRY(cudaMemcpyAsync(v.sc, &init, sizeof(init), cudaMemcpyHostToDevice, s));
-    SB_TRY(cudaMemsetAsync(b->bar, 0, sizeof(GridBarrier), s));
+    SB_TRY(cudaMemsetAsync(b->bar, 0, kBarrierClear, s));
     SB_TRY(b->fused ? launch_grid_cg_fused(v, (int)b->opts.dot, b->bar, b->rec, s)
                     : launch_grid_cg(v, (int)b->opts.dot, b->bar, s));
     k_sb_from_planes<<<blocks_for(v.n), kBlock, 0, s>>>(v.dv, b->dev.sell_inv, b->cs.x, v.n);

@@ -161,6 +161,7 @@ int build_topology(uint32_t n, const float* X, uint32_t t, const uint32_t* tris,
     c.row_ptr.assign(n + 1, 0);
     c.row_cols.clear();
     c.max_deg = 0;
+    c.band = 0;
     for (uint32_t i = 0; i < n; ++i) {
         auto& v = nb[i];
         std::sort(v.begin() + 1, v.end());
@@ -169,6 +170,7 @@ int build_topology(uint32_t n, const float* X, uint32_t t, const uint32_t* tris,
         v.erase(std::remove(v.begin() + 1, v.end(), i), v.end());
         if (v.size() > kMaxDegree) return kUnsupported;
         c.max_deg = std::max<uint32_t>(c.max_deg, (uint32_t)v.size());
+        if (v.size() > 1) c.band = std::max(c.band, std::max(v[1] < i ? i - v[1] : 0u, v.back() > i ? v.back() - i : 0u));
         c.row_cols.insert(c.row_cols.end(), v.begin(), v.end());
         c.row_ptr[i + 1] = (uint32_t)c.row_cols.size();
     }

@@ -36,6 +36,7 @@ struct ClothTopology {
     std::vector<uint32_t> row_ptr;           // n + 1
     std::vector<uint32_t> row_cols;
     uint32_t max_deg = 0;
+    uint32_t band = 0;                       // widest |row - column|
     // SELL-32
     uint32_t nslices = 0, E = 0;
     std::vector<uint32_t> slice_off;         // nslices + 1

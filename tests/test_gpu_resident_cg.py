@@ -1,0 +1,63 @@
+"""The on-chip CG of one cloth against the per-iteration kernels: the same
+rows, so with FP64 dots the same floats but for the sums' last bits.
+
+Sizes sit on the edges of its shapes: one CTA (up to 256 rows), clusters (a
+last CTA with few rows or none, 4,096 rows), the grid (one and two rows a
+thread, blocks that do not all fit), and a coupling across the whole cloth
+(sewn panels)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(b3g, kind, side):
+    if kind == "sewn":
+        return b3g.sewn_scene(side)
+    if kind == "bend":
+        return b3g.sphere_scene(side)
+    return b3g.plain_scene(side)
+
+
+@pytest.mark.parametrize("kind,side", [("plain", 2), ("plain", 6), ("bend", 16), ("plain", 17), ("bend", 33),
+                                       ("plain", 64), ("plain", 65), ("sewn", 9), ("sewn", 45), ("sewn", 50),
+                                       ("bend", 67), ("bend", 250), ("plain", 280), ("plain", 384)])
+@pytest.mark.parametrize("dot", [0, 1, 2])
+def test_on_chip_cg_matches_launches(b3g, kind, side, dot):
+    """x of an iteration differs only by the rounding of alpha and beta, one
+    float rounding (6e-8) each and iteration, magnified by at most the CG's own
+    sensitivity; 8 iterations of both from the same system stay within 1e-5 of
+    the largest entry (FP64 sums: within 1e-6)."""
+    scene = _scene(b3g, kind, side)
+    opts = b3g.SolverOptions(b3g.STOP_RELATIVE, 1e-9, 3 if side == 2 else 8, dot)
+    rng = np.random.default_rng(side)
+    v = rng.normal(0.0, 0.1, (scene.mesh.vertex_count, 3)).astype(np.float32)
+    v[np.asarray(scene.pinned, np.int64)] = 0.0
+    got = []
+    for persistent in (False, True):
+        cloth = b3g.Cloth(scene.mesh, scene.cdef).setup(scene, opts)
+        cloth.set_cg_strategy(persistent)
+        cloth.write_state(v=v, dv=0.1 * v)
+        out = cloth.step_profiled(scene.dt)
+        got.append((out["iterations"], cloth.state()["dv"]))
+        again = cloth.step(scene.dt)
+        assert again["iterations"] > 0
+    assert got[0][0] == got[1][0]
+    a, b = got[0][1].astype(np.float64), got[1][1].astype(np.float64)
+    assert np.abs(a - b).max() <= (1e-6 if dot == 2 else 1e-5) * np.abs(a).max()
+
+
+def test_on_chip_cg_repeats_itself(b3g):
+    """The grid form's sums run in a fixed order: the same step twice gives the
+    same bits."""
+    scene = b3g.plain_scene(128)
+    cloth = b3g.Cloth(scene.mesh, scene.cdef).setup(scene, b3g.SolverOptions.relative(1e-4, 50, b3g.DOT_F32))
+    cloth.set_cg_strategy(True)
+    x0 = cloth.state()
+    runs = []
+    for _ in range(3):
+        cloth.write_state(x0["x"], x0["v"], x0["dv"])
+        cloth.step(scene.dt)
+        cloth.step(scene.dt)
+        runs.append(cloth.state()["dv"])
+    assert all(np.array_equal(runs[0], r) for r in runs[1:])
