@@ -584,7 +584,8 @@ class Cloth:
 
     def set_cg_strategy(self, persistent, fused: bool = False) -> None:
         """False: per-iteration launches in a graph loop; True: one persistent
-        cooperative launch (fused: one grid reduction per iteration)."""
+        cooperative launch (fused: one grid reduction per iteration).  A cloth
+        that fits on chip is solved there in one launch (b3g.h)."""
         code = 0 if not persistent else 2 if fused else 1
         check(lib().b3g_cloth_set_cg_strategy(self.h, code), "set_cg_strategy")
 

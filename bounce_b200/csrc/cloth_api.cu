@@ -104,7 +104,21 @@ void destroy_graph(b3g_cloth* c)
     c->exec = nullptr;
 }
 
-bool persistent_cg(const b3g_cloth* c) { return c->cg_strategy != B3G_CG_LAUNCHES; }
+// The on-chip shape of the cloth's solve, if it runs there: any cloth that
+// fits under the persistent strategies, one that fits a cluster under all.
+// A snapshot written, its frames and the state read, per-iteration launches
+// against one launch: 8^2 (1 frame) 453 and 156 us, 32^2 (4 frames) 1,007 and
+// 426 us, two sewn panels of 45^2 (4 frames) 1,815 and 662 us.  The fused
+// form's one reduction saves nothing on chip: 383^2 (2 frames) 2,019 and
+// 1,807 us.
+ResShape on_chip(const b3g_cloth* c)
+{
+    const ResShape s = resident_shape(c->dev);
+    return s.grid && c->cg_strategy == B3G_CG_LAUNCHES ? ResShape() : s;
+}
+
+// Whether the whole CG is one launch.
+bool persistent_cg(const b3g_cloth* c) { return c->cg_strategy != B3G_CG_LAUNCHES || on_chip(c).ctas; }
 
 // The fused CG's record buffer, sized for the cloth's current vertex count
 // (a new layout changes it; a captured graph holding the old one is dropped).
@@ -120,11 +134,12 @@ b3g_status ensure_cg_rec(b3g_cloth* c)
     return B3G_OK;
 }
 
-// The persistent CG of the cloth's strategy: the barrier is cleared, then one
-// cooperative launch (two grid reductions per iteration, or the fused form).
+// The CG of the cloth in one launch: on chip where it fits, else the
+// barrier is cleared and a cooperative launch runs the cloth's strategy (two
+// grid reductions per iteration, or the fused form).
 cudaError_t launch_persistent_cg(b3g_cloth* c, int dot, cudaStream_t st)
 {
-    const ResShape shape = c->cg_strategy == B3G_CG_PERSISTENT ? resident_shape(c->dev) : ResShape();
+    const ResShape shape = on_chip(c);
     if (shape.ctas) return launch_resident_cg(c->dev, shape, dot, st);
     cudaError_t e = cudaMemsetAsync(c->dev.bar, 0, kBarrierClear, st);
     if (e != cudaSuccess) return e;

@@ -88,7 +88,7 @@ ResShape resident_shape(const ClothDev& c)
         r.threads = 32u * ((per + r.rows_per_thread - 1u) / r.rows_per_thread);
         // threads without rows of their own help with the halo
         const uint32_t halo = std::min(n, r.chunk + 2u * c.band) - std::min(n, r.chunk);
-        const uint32_t most = grid || ctas == 1u ? (uint32_t)kResMaxThreads : 32u * kResTeamWarps;
+        const uint32_t most = (uint32_t)kResMaxThreads;
         r.threads = std::max(r.threads, std::min(most, 32u * ((halo + 32u * kResHalo - 1u) / (32u * kResHalo))));
         if (grid) r.threads = std::max(r.threads, 32u * ((r.ctas + 31u) / 32u));  // a thread a partial
         r.wide = halo > (uint32_t)kResHalo * r.threads;
@@ -129,10 +129,6 @@ cudaError_t launch_resident_cg(const ClothDev& c, const ResShape& s, int dot, cu
         attr[0].id = cudaLaunchAttributeCooperative;
         attr[0].val.cooperative = 1;
     } else {
-        if (s.ctas > 8) {
-            e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            if (e != cudaSuccess) return e;
-        }
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = s.ctas;
         attr[0].val.clusterDim.y = 1;

@@ -49,13 +49,12 @@ constexpr uint32_t kResTimeout = 7;  // B3G_ERR_TIMEOUT
 
 // The fixed part of the shared memory.
 struct ResShared {
-    double wsum[2][2][kResMaxTeam * kResTeamWarps];  // [parity][value][rank and warp]
+    double wsum[2][2][kResMaxWords];  // [parity][value][warp of the team]
     unsigned long long mbar;
     int lost;
     uint32_t listed;  // wide windows: halo rows the CTA's rows touch
 };
 static_assert(sizeof(ResShared) <= kResHeader, "fixed shared memory of the resident CG");
-static_assert(kResMaxWarps <= kResMaxTeam * kResTeamWarps, "a CTA alone keeps every warp's sum");
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -84,8 +83,9 @@ __device__ __forceinline__ typename D::T warp_sum(typename D::T v)
     return v;
 }
 
-// The sum of `count` 8-byte words in shared memory, in a fixed tree, by one
-// thread: no shuffles.
+// The sum of up to 16 8-byte words in shared memory by one thread, in the
+// order of block_reduce and grid_reduce (cg_common.cuh) over blocks of eight
+// warps: a tree over each eight, then the two.
 template <class D>
 __device__ __forceinline__ typename D::T words_sum(const double* w, uint32_t count)
 {
@@ -95,16 +95,45 @@ __device__ __forceinline__ typename D::T words_sum(const double* w, uint32_t cou
     for (uint32_t k = 0; k < (uint32_t)kResMaxWarps; ++k)
         a[k] = k < count ? *reinterpret_cast<const T*>(w + k) : D::zero();
 #pragma unroll
-    for (int step = kResMaxWarps / 2; step > 0; step >>= 1)
+    for (int step = 4; step > 0; step >>= 1)
 #pragma unroll
-        for (int k = 0; k < step; ++k) a[k] = D::combine(a[k], a[k + step]);
-    return a[0];
+        for (int k = 0; k < step; ++k) {
+            a[k] = D::combine(a[k], a[k + step]);
+            a[k + 8] = D::combine(a[k + 8], a[k + 8 + step]);
+        }
+    return D::combine(a[0], a[8]);
+}
+
+// The same order for up to 128 words, by a warp: the sum in lane 0.
+template <class D>
+__device__ __forceinline__ typename D::T words_sum_warp(const double* w, uint32_t count)
+{
+    typedef typename D::T T;
+    const uint32_t lane = threadIdx.x & 31u;
+    T a[kResMaxWords / 32];
+#pragma unroll
+    for (uint32_t m = 0; m < (uint32_t)kResMaxWords / 32u; ++m) {
+        const uint32_t i = lane + 32u * m;
+        a[m] = i < count ? *reinterpret_cast<const T*>(w + i) : D::zero();
+        if (32u * m < count)
+#pragma unroll
+            for (int off = 4; off > 0; off >>= 1) a[m] = D::combine(a[m], D::shfl(a[m], off));
+    }
+    // blocks 4 m + lane / 8: a tree over sixteen
+    if (count > 32u) {
+        a[0] = D::combine(a[0], a[2]);
+        a[1] = D::combine(a[1], a[3]);
+        a[0] = D::combine(a[0], a[1]);
+    }
+    a[0] = D::combine(a[0], D::shfl(a[0], 16));
+    return D::combine(a[0], D::shfl(a[0], 8));
 }
 
 // One CTA (size 1) or the CTAs of a thread-block cluster.
 struct TeamScope {
     static constexpr bool kGrid = false;
     uint32_t rank, size, parity;
+    uint32_t word, words;  // this warp's word of the sums (kResMaxWords: none), and how many there are
     ResShared* sh;
     float* zs;  // 3 planes of `chunk`: z of this CTA's rows, read by the team
 
@@ -122,13 +151,13 @@ struct TeamScope {
     __device__ bool sum(typename D::T (&v)[NV])
     {
         typedef typename D::T T;
-        const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        const uint32_t lane = threadIdx.x & 31u;
         parity ^= 1u;
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             const unsigned long long u = __shfl_sync(0xffffffffu, pack8(warp_sum<D>(v[k])), 0);
-            double* mine = &sh->wsum[parity][k][rank * nw + warp];
-            if (lane < size) {
+            double* mine = &sh->wsum[parity][k][word];
+            if (lane < size && word < (uint32_t)kResMaxWords) {
                 double* to = size == 1 ? mine : rcg::this_cluster().map_shared_rank(mine, lane);
                 *reinterpret_cast<unsigned long long*>(to) = u;
             }
@@ -137,13 +166,8 @@ struct TeamScope {
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             const double* w = sh->wsum[parity][k];
-            if (size * nw <= (uint32_t)kResMaxWarps) {
-                v[k] = words_sum<D>(w, size * nw);
-            } else {
-                T a = D::zero();
-                for (uint32_t i = lane; i < size * nw; i += 32u) a = D::combine(a, *reinterpret_cast<const T*>(w + i));
-                v[k] = unpack8<T>(__shfl_sync(0xffffffffu, pack8(warp_sum<D>(a)), 0));
-            }
+            if (words <= (uint32_t)kResMaxWarps) v[k] = words_sum<D>(w, words);
+            else v[k] = unpack8<T>(__shfl_sync(0xffffffffu, pack8(words_sum_warp<D>(w, words)), 0));
         }
         return true;
     }
@@ -439,6 +463,12 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
     float* As = reinterpret_cast<float*>(smem + a_off);
     const uint32_t q0 = r0 >> 5, q1 = empty ? q0 : (r1 + 31u) >> 5;
     const uint32_t so0 = c.slice_off[q0];
+    if constexpr (!S::kGrid) {
+        // one row a thread: a word a slice, summed in the order of the
+        // per-iteration kernels (their FP32 sums come out the same)
+        team.word = RPT > 1 ? team.rank * nw + warp : q0 + warp < q1 ? q0 + warp : (uint32_t)kResMaxWords;
+        team.words = RPT > 1 ? team.size * nw : (n + 31u) >> 5;
+    }
     const uint32_t room = (smem_bytes - a_off) / 36u;  // blocks
 
     // the resident slices: the first ones that fit

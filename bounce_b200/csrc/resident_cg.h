@@ -11,13 +11,13 @@
 namespace b3g {
 
 constexpr int kResMaxThreads = 512;
-constexpr int kResMaxTeam = 16;   // CTAs of a cluster
+constexpr int kResMaxTeam = 8;    // CTAs of a cluster
 constexpr int kResMaxGrid = 160;  // CTAs of a cooperative launch
 constexpr int kResSlots = 16;     // widest row
-constexpr int kResTeamWarps = 16; // warps of a CTA of a cluster
+constexpr int kResMaxWords = 128; // warps of a team
 constexpr int kResLine = 8;       // 16-byte words between two partials of a grid
 constexpr int kResHalo = 4;       // halo rows a thread
-constexpr uint32_t kResHeader = 8320;
+constexpr uint32_t kResHeader = 4224;
 constexpr uint32_t kResSmemLimit = 227 * 1024;
 
 // Rows whose direction a CTA of `chunk` rows keeps: its own and the band's.

@@ -269,11 +269,15 @@ b3g_status b3g_cloth_apply_translations(b3g_cloth* cloth, const float* translati
 b3g_status b3g_cloth_step(b3g_cloth* cloth, float dt, uint32_t velocity_iterations,
                           uint32_t position_iterations, b3g_step_stats* stats);
 
-/* How one cloth's CG runs on the GPU.  LAUNCHES (default): three kernels
- * per iteration inside a CUDA-graph while loop.  PERSISTENT: one cooperative
- * launch for the whole solve, two grid reductions per iteration, separated by
- * grid barriers with bounded waits (B3G_ERR_TIMEOUT if one gives up); for
- * large cloths.  PERSISTENT_FUSED: as PERSISTENT with one grid reduction per
+/* How one cloth's CG runs on the GPU.  A cloth whose system fits on chip
+ * (rows of at most 16 blocks, couplings within a band of vertex numbers that
+ * a CTA can hold) is solved there in one launch, with the same arithmetic: up
+ * to 4,096 vertices by one CTA or cluster under every strategy, up to about
+ * 150,000 by a cooperative launch under the persistent ones (bounded waits,
+ * B3G_ERR_TIMEOUT if one gives up).  Otherwise: LAUNCHES (default): three
+ * kernels per iteration inside a CUDA-graph while loop.  PERSISTENT: one
+ * cooperative launch for the whole solve, two grid reductions per iteration,
+ * separated by grid barriers with bounded waits; for large cloths.  PERSISTENT_FUSED: as PERSISTENT with one grid reduction per
  * iteration.  Each vertex publishes r, s and p once per iteration, and every
  * row forms its neighbours' next direction from them.  The reduction returns
  * p.s, s.z, s.P^-1 s and r.z (z = S P^-1 r) of the iterate: alpha = r.z / p.s
