@@ -76,6 +76,7 @@ struct b3g_server {
     std::mutex mu;
     std::condition_variable cv;
     std::deque<Request*> prep;
+    size_t preparing = 0;                    // taken by a worker, not ready yet
     std::vector<std::thread> workers;
     bool stop = false;
 
@@ -116,6 +117,7 @@ void worker_main(b3g_server* s)
             if (s->stop && s->prep.empty()) return;
             r = s->prep.front();
             s->prep.pop_front();
+            s->preparing += 1;
         }
         b3g_mesh_desc m{(uint32_t)(r->verts.size() / 3), r->verts.data(), (uint32_t)(r->tris.size() / 3),
                         r->tris.data(), 0, nullptr};
@@ -125,6 +127,7 @@ void worker_main(b3g_server* s)
         // HBM budget then admits more of them
         b3g_status st = prepare_cloth(&m, &r->def, &c, false);
         std::lock_guard<std::mutex> lk(s->mu);
+        s->preparing -= 1;
         if (st != B3G_OK) {
             r->status = st;
             r->state = R_FAILED;
@@ -389,7 +392,7 @@ b3g_status b3g_server_tick(b3g_server* s, double now, b3g_server_tick_info* info
             s->used += r->bytes;
             newly.push_back(r);
         }
-        ti.queued = (uint32_t)(s->prep.size() + s->ready.size());
+        ti.queued = (uint32_t)(s->prep.size() + s->preparing + s->ready.size());
     }
     const auto ta = std::chrono::steady_clock::now();
     std::vector<Request*> joined;
@@ -527,7 +530,7 @@ b3g_status b3g_server_stats(const b3g_server* cs, b3g_server_statistics* out)
     out->completed = s->completed;
     out->rejected = s->rejected;
     out->active = (uint32_t)s->active.size();
-    out->queued = (uint32_t)(s->prep.size() + s->ready.size());
+    out->queued = (uint32_t)(s->prep.size() + s->preparing + s->ready.size());
     out->peak_active = s->peak_active;
     out->peak_bytes = s->peak_used;
     // step latency percentiles: every cloth stepped in a tick waited that tick

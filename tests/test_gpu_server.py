@@ -99,3 +99,21 @@ def test_oversized_request_is_rejected(b3g):
         time.sleep(0.01)
     info = srv.poll(rid)
     assert info["state"] == 4 and info["status"] == 8  # failed, capacity
+
+
+def test_request_in_preparation_counts_as_queued(b3g):
+    """From its submission to its last step a request is queued or active:
+    drain() does not return while a worker still prepares one."""
+    srv = b3g.Server(budget_bytes=2 * 10**9, max_active=4, host_threads=1)
+    scene = b3g.plain_scene(160)
+    for _ in range(5):
+        rid = srv.submit_scene(scene, 1)
+        while srv.poll(rid)["state"] < 2:
+            st = srv.stats()
+            assert st["queued"] + st["active"] >= 1
+            if st["queued"] and srv.poll(rid)["state"] == 1:
+                srv.tick()
+        srv.drain()
+        assert srv.poll(rid)["state"] == 3
+        srv.release(rid)
+    srv.close()
