@@ -22,5 +22,9 @@ struct BatchCgArgs {
 // they differ (each cloth's own setting is then read on the device).
 cudaError_t launch_batch_cg(const BatchCgArgs& a, int team, int dot, int grid_blocks, cudaStream_t st);
 int batch_team_max_blocks(int team, int dot);
+// Whether cloth c is solved on chip by a team of `team` CTAs, and the launch
+// over such cloths (batch_resident.cu).
+bool batch_on_chip(const ClothDev& c, int team);
+cudaError_t launch_batch_resident(const BatchCgArgs& a, int team, int dot, cudaStream_t st);
 
 }  // namespace b3g

@@ -87,6 +87,7 @@ struct b3g_batch {
     uint32_t graph_pi = UINT32_MAX, graph_sched = 0;
     uint32_t graph_hulls = 0;  // whether the graph holds the hull contact kernel
     uint32_t graph_kernels = 0;
+    uint32_t nchip = 0;  // the first tasks: cloths solved on chip
     uint32_t ntasks = 0, total_rows = 0, max_deg = 0;
     uint32_t total_elems = 0;  // triangles, springs and mouse forces of every cloth
     uint32_t hulls = 0;  // some cloth of the batch has a hull collider
@@ -145,31 +146,49 @@ void plan(b3g_batch* b, b3g_cloth* const* cloths, uint32_t count)
     std::stable_sort(idx.begin(), idx.end(), [&](uint32_t a, uint32_t c) { return work(a) > work(c); });
     const uint32_t T = b->sched.cluster;
     uint32_t w = 0, nt = 0;
-    std::vector<uint32_t> small;
-    for (uint32_t k : idx) {
-        const bool split = T > 1 && b->sched.split_class[size_class(cloths[k]->dev.n)] != 0;
-        if (split) {
-            b->h_order[w] = k;
-            b->h_tasks[nt++] = make_uint2(w, 0u);
-            ++w;
-        } else {
-            small.push_back(k);
+    auto is_split = [&](uint32_t k) { return T > 1 && b->sched.split_class[size_class(cloths[k]->dev.n)] != 0; };
+    // the cloths that fit their team's shared memory run on chip, in a launch
+    // ahead of the others'
+    auto on_chip = [&](uint32_t k) { return batch_on_chip(cloths[k]->dev, is_split(k) ? (int)T : 1); };
+    for (int chip = 1; chip >= 0; --chip) {
+        std::vector<uint32_t> small;
+        for (uint32_t k : idx) {
+            if ((on_chip(k) ? 1 : 0) != chip) continue;
+            if (is_split(k)) {
+                b->h_order[w] = k;
+                b->h_tasks[nt++] = make_uint2(w, 0u);
+                ++w;
+            } else {
+                small.push_back(k);
+            }
         }
-    }
-    for (size_t q = 0; q < small.size(); q += T) {
-        const uint32_t cnt = (uint32_t)std::min<size_t>(T, small.size() - q);
-        b->h_tasks[nt++] = make_uint2(w, cnt);
-        for (uint32_t r = 0; r < cnt; ++r) b->h_order[w++] = small[q + r];
+        for (size_t q = 0; q < small.size(); q += T) {
+            const uint32_t cnt = (uint32_t)std::min<size_t>(T, small.size() - q);
+            b->h_tasks[nt++] = make_uint2(w, cnt);
+            for (uint32_t r = 0; r < cnt; ++r) b->h_order[w++] = small[q + r];
+        }
+        if (chip) b->nchip = nt;
     }
     b->ntasks = nt;
     b->assemble_block = 0;  // chosen at launch for occupancy
+}
+
+// The CG of every planned cloth: on chip, then the others.
+cudaError_t launch_cg(b3g_batch* b, cudaStream_t st)
+{
+    cudaError_t e = cudaMemsetAsync(b->d_next, 0, 256, st);
+    if (e != cudaSuccess) return e;
+    const int T = (int)b->sched.cluster;
+    const BatchCgArgs chip{b->d_descs, b->d_order, b->d_tasks, b->nchip, b->d_next};
+    const BatchCgArgs rest{b->d_descs, b->d_order, b->d_tasks + b->nchip, b->ntasks - b->nchip, b->d_next + 32};
+    if ((e = launch_batch_resident(chip, T, b->dot, st)) != cudaSuccess) return e;
+    return launch_batch_cg(rest, T, b->dot, 0, st);
 }
 
 b3g_status enqueue(b3g_batch* b, uint32_t count, uint32_t pi, cudaStream_t st, uint32_t* kernels)
 {
     RowSpan sp{b->d_descs, b->d_prefix, count, b->total_rows, b->max_deg, b->hulls, b->slot_asm,
                        b->d_prefix + count + 1, b->total_elems};
-    BatchCgArgs a{b->d_descs, b->d_order, b->d_tasks, b->ntasks, b->d_next};
     uint32_t k = 0;
     B3G_TRY(cudaMemcpyAsync(b->d_descs, b->h_descs, count * sizeof(ClothDev), cudaMemcpyHostToDevice, st));
     B3G_TRY(cudaMemcpyAsync(b->d_stage, b->h_stage, count * sizeof(StepScalars), cudaMemcpyHostToDevice, st));
@@ -182,17 +201,16 @@ b3g_status enqueue(b3g_batch* b, uint32_t count, uint32_t pi, cudaStream_t st, u
     B3G_TRY(cudaGetLastError());
     B3G_TRY(launch_span_contacts_update(sp, st));
     B3G_TRY(launch_span_assemble(sp, b->assemble_block, st));
-    B3G_TRY(cudaMemsetAsync(b->d_next, 0, sizeof(uint32_t), st));
     // under stream capture the records must be external to become event
     // nodes, so that the CG launch is timed on every replay of the graph
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     B3G_TRY(cudaStreamIsCapturing(st, &cap));
     const unsigned rec_flags = cap == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
     B3G_TRY(cudaEventRecordWithFlags(b->ev_cg0, st, rec_flags));
-    B3G_TRY(launch_batch_cg(a, (int)b->sched.cluster, b->dot, 0, st));
+    B3G_TRY(launch_cg(b, st));
     B3G_TRY(cudaEventRecordWithFlags(b->ev_cg1, st, rec_flags));
     B3G_TRY(launch_span_finalize(sp, st));
-    k += 4;
+    k += 3 + (b->nchip ? 1u : 0u) + (b->nchip < b->ntasks ? 1u : 0u);
     for (uint32_t it = 1; it < pi && it < (uint32_t)kMaxPosIters; ++it) {
         B3G_TRY(launch_span_contact_position(sp, it, st));
         ++k;
@@ -493,7 +511,6 @@ b3g_status b3g_batch_autotune(b3g_batch* b, b3g_cloth* const* cloths, uint32_t c
             plan(b, cloths, count);
             RowSpan sp{b->d_descs, b->d_prefix, count, b->total_rows, b->max_deg, b->hulls, b->slot_asm,
                        b->d_prefix + count + 1, b->total_elems};
-            BatchCgArgs a{b->d_descs, b->d_order, b->d_tasks, b->ntasks, b->d_next};
             B3G_TRY(cudaMemcpyAsync(b->d_descs, b->h_descs, count * sizeof(ClothDev), cudaMemcpyHostToDevice, st));
             B3G_TRY(cudaMemcpyAsync(b->d_stage, b->h_stage, count * sizeof(StepScalars), cudaMemcpyHostToDevice, st));
             B3G_TRY(cudaMemcpyAsync(b->d_prefix, b->h_prefix, 2 * (count + 1) * 4, cudaMemcpyHostToDevice, st));
@@ -504,9 +521,8 @@ b3g_status b3g_batch_autotune(b3g_batch* b, b3g_cloth* const* cloths, uint32_t c
             B3G_TRY(launch_span_assemble(sp, b->assemble_block, st));
             float bestrun = 1e30f;
             for (int rep = 0; rep < 3; ++rep) {
-                B3G_TRY(cudaMemsetAsync(b->d_next, 0, 4, st));
                 B3G_TRY(cudaEventRecord(b->ev0, st));
-                B3G_TRY(launch_batch_cg(a, (int)sc.cluster, b->dot, 0, st));
+                B3G_TRY(launch_cg(b, st));
                 B3G_TRY(cudaEventRecord(b->ev1, st));
                 B3G_TRY(cudaEventSynchronize(b->ev1));
                 float ms = 0.0f;

@@ -9,7 +9,7 @@ namespace b3g {
 
 namespace {
 
-template <int DOT, int RPT>
+template <int DOT, int RPT, int SLOTS>
 __global__ void __launch_bounds__(kResMaxThreads, 1)
     k_resident_team(const __grid_constant__ ClothDev c, uint32_t chunk, uint32_t wide, uint32_t smem_bytes)
 {
@@ -23,11 +23,11 @@ __global__ void __launch_bounds__(kResMaxThreads, 1)
     team.zs = reinterpret_cast<float*>(smem + kResHeader) + 3u * (size_t)res_window(c.n, chunk, c.band);
     uint32_t phase = 0u;
     res_init_copy_barrier(sh);
-    resident_solve<DOT, RPT>(c, team, smem, chunk, wide != 0u, smem_bytes, phase);
+    resident_solve<DOT, RPT, SLOTS>(c, team, smem, chunk, wide != 0u, smem_bytes, phase);
     team.barrier();  // no CTA leaves while another may still write into it
 }
 
-template <int DOT, int RPT>
+template <int DOT, int RPT, int SLOTS>
 __global__ void __launch_bounds__(kResMaxThreads, 1)
     k_resident_grid(const __grid_constant__ ClothDev c, uint32_t chunk, uint32_t wide, uint32_t smem_bytes)
 {
@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1)
     team.arrivals = *(volatile uint32_t*)&c.bar->arrivals;
     uint32_t phase = 0u;
     res_init_copy_barrier(sh);
-    const bool good = resident_solve<DOT, RPT>(c, team, smem, chunk, wide != 0u, smem_bytes, phase);
+    const bool good = resident_solve<DOT, RPT, SLOTS>(c, team, smem, chunk, wide != 0u, smem_bytes, phase);
     if (threadIdx.x == 0 && !good) {
         c.sc->status = kResTimeout;
         c.sc->cont = 0;
@@ -60,12 +60,16 @@ __global__ void __launch_bounds__(kResMaxThreads, 1)
     }
 }
 
-template <int DOT>
-const void* kernel_for(bool grid, uint32_t rpt)
+template <int DOT, int RPT, int SLOTS>
+const void* kernel_of(bool grid)
 {
-    if (grid)
-        return rpt == 1 ? (const void*)k_resident_grid<DOT, 1> : (const void*)k_resident_grid<DOT, 2>;
-    return rpt == 1 ? (const void*)k_resident_team<DOT, 1> : (const void*)k_resident_team<DOT, 2>;
+    return grid ? (const void*)k_resident_grid<DOT, RPT, SLOTS> : (const void*)k_resident_team<DOT, RPT, SLOTS>;
+}
+template <int DOT>
+const void* kernel_for(bool grid, uint32_t rpt, bool few)
+{
+    if (rpt == 1) return kernel_of<DOT, 1, kResSlots>(grid);
+    return few ? kernel_of<DOT, 2, kResFewSlots>(grid) : kernel_of<DOT, 2, kResSlots>(grid);
 }
 
 }  // namespace
@@ -87,11 +91,11 @@ ResShape resident_shape(const ClothDev& c)
         r.rows_per_thread = r.chunk <= (uint32_t)kResMaxThreads ? 1u : 2u;
         r.threads = 32u * ((per + r.rows_per_thread - 1u) / r.rows_per_thread);
         // threads without rows of their own help with the halo
-        const uint32_t halo = std::min(n, r.chunk + 2u * c.band) - std::min(n, r.chunk);
+        const uint32_t halo = res_window(n, r.chunk, c.band) - std::min(n, r.chunk);
         const uint32_t most = (uint32_t)kResMaxThreads;
         r.threads = std::max(r.threads, std::min(most, 32u * ((halo + 32u * kResHalo - 1u) / (32u * kResHalo))));
         if (grid) r.threads = std::max(r.threads, 32u * ((r.ctas + 31u) / 32u));  // a thread a partial
-        r.wide = halo > (uint32_t)kResHalo * r.threads;
+        r.wide = res_wide(n, r.chunk, c.band, r.threads);
         const uint64_t off = res_block_offset(n, r.chunk, c.band, !grid && ctas > 1u, r.wide);
         const uint64_t all = off + (uint64_t)r.chunk * c.max_deg * 36u;
         r.smem = (uint32_t)std::min<uint64_t>(all, kResSmemLimit);
@@ -115,8 +119,10 @@ ResShape resident_shape(const ClothDev& c)
 
 cudaError_t launch_resident_cg(const ClothDev& c, const ResShape& s, int dot, cudaStream_t st)
 {
-    const void* fn = dot == 2 ? kernel_for<2>(s.grid, s.rows_per_thread)
-                   : dot == 1 ? kernel_for<1>(s.grid, s.rows_per_thread) : kernel_for<0>(s.grid, s.rows_per_thread);
+    const bool few = c.max_deg <= (uint32_t)kResFewSlots;
+    const void* fn = dot == 2 ? kernel_for<2>(s.grid, s.rows_per_thread, few)
+                   : dot == 1 ? kernel_for<1>(s.grid, s.rows_per_thread, few)
+                              : kernel_for<0>(s.grid, s.rows_per_thread, few);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemLimit);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};

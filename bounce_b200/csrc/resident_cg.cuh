@@ -10,7 +10,8 @@
 //    of them (band = the widest |row - column| of the matrix), so a product
 //    gathers p from shared memory only.
 // x, r, z, p and P^-1 of its own rows and their column indices stay in
-// registers.  Per iteration only z of the window's halo crosses CTAs: the
+// registers (with more than two rows a thread, x and P^-1 in L2, z in shared memory
+// and p in its window).  Per iteration only z of the window's halo crosses CTAs: the
 // halo's p = z + beta p_old is formed where it is needed, from the same float
 // expression as its owner's.
 //
@@ -342,11 +343,12 @@ struct StopBound {
 };
 
 // One row: its blocks' first word (in the resident blocks or in ClothDev::vals),
-// the distance of their components, its slice's width, and the window indices
-// of its columns, two a word.
+// its slice's width, and the window indices of its columns, two a word.
+template <int SLOTS>
 struct ResRow {
-    uint32_t off, cs, width;
-    uint32_t col[kResSlots / 2];
+    static constexpr int kSlots = SLOTS;
+    uint32_t off, width;
+    uint32_t col[SLOTS / 2];
 };
 
 template <int I>
@@ -381,8 +383,8 @@ __device__ __forceinline__ void stp(float* P, uint32_t j, f3 v)
 // The blocks and directions of slots K .. K + G - 1, then their products in
 // slot order, acc = acc + A_k p_k (b3Mat33 * b3Vec3, include/bounce/common/
 // math/mat33.h:129-132): the loads of the G slots are in flight together.
-template <int K, int G, class A>
-__device__ __forceinline__ f3 res_slots(f3 acc, const ResRow& r, const A (&a)[9], const float* P)
+template <int K, int G, class R, class A>
+__device__ __forceinline__ f3 res_slots(f3 acc, const R& r, const A (&a)[9], const float* P)
 {
     m3 m[G];
     f3 p[G];
@@ -402,38 +404,43 @@ __device__ __forceinline__ f3 res_slots(f3 acc, const ResRow& r, const A (&a)[9]
 }
 
 // s_i = sum_k A_k p_k of one row.  The warp walks its slice's width (a row's
-// padding holds zero blocks on the diagonal's column): fours, then a pair and
-// a single slot.
-template <int K, class A>
-__device__ __forceinline__ f3 res_walk(f3 acc, const ResRow& r, const A (&a)[9], const float* P)
+// padding holds zero blocks on the diagonal's column): fours where one row a
+// thread leaves the registers for them (spills would go to L2: shared memory
+// takes nearly all of L1), then a pair and a single slot.
+template <int G, int K, class R, class A>
+__device__ __forceinline__ f3 res_walk(f3 acc, const R& r, const A (&a)[9], const float* P)
 {
-    if constexpr (K < kResSlots) {
-        if (K + 4u <= r.width) {
-            acc = res_slots<K, 4>(acc, r, a, P);
-            return res_walk<K + 4>(acc, r, a, P);
+    if constexpr (K < R::kSlots) {
+        if (K + (uint32_t)G <= r.width) {
+            acc = res_slots<K, G>(acc, r, a, P);
+            return res_walk<G, K + G>(acc, r, a, P);
         }
-        if (K + 2u <= r.width) {
-            acc = res_slots<K, 2>(acc, r, a, P);
-            if (K + 3u == r.width) acc = res_slots<K + 2, 1>(acc, r, a, P);
-        } else if (K + 1u == r.width) {
-            acc = res_slots<K, 1>(acc, r, a, P);
+        if constexpr (G > 2) {
+            if (K + 2u <= r.width) {
+                acc = res_slots<K, 2>(acc, r, a, P);
+                if (K + 3u == r.width) acc = res_slots<K + 2, 1>(acc, r, a, P);
+                return acc;
+            }
         }
+        if (K + 1u == r.width) acc = res_slots<K, 1>(acc, r, a, P);
     }
     return acc;
 }
-__device__ __forceinline__ f3 res_row_times(const ResRow& r, uint32_t blocks, const float* P)
+template <int G, class R>
+__device__ __forceinline__ f3 res_row_times(const R& r, uint32_t blocks, const float* P)
 {
     uint32_t a[9];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) a[q] = blocks + 4u * (r.off + q * r.cs);
-    return res_walk<0>(zero3(), r, a, P);
+    for (int q = 0; q < 9; ++q) a[q] = blocks + 4u * (r.off + q * 32u * r.width);
+    return res_walk<G, 0>(zero3(), r, a, P);
 }
-__device__ __forceinline__ f3 res_row_times(const ResRow& r, const float* blocks, const float* P)
+template <int G, class R>
+__device__ __forceinline__ f3 res_row_times(const R& r, const float* blocks, uint32_t plane, const float* P)
 {
     const float* a[9];
 #pragma unroll
-    for (int q = 0; q < 9; ++q) a[q] = blocks + r.off + (size_t)q * r.cs;
-    return res_walk<0>(zero3(), r, a, P);
+    for (int q = 0; q < 9; ++q) a[q] = blocks + r.off + (size_t)q * plane;
+    return res_walk<G, 0>(zero3(), r, a, P);
 }
 
 // The whole solve by a team.  `smem`: kResHeader bytes (the scope's
@@ -443,12 +450,14 @@ __device__ __forceinline__ f3 res_row_times(const ResRow& r, const float* blocks
 // its rows touch.  `phase`: the copy barrier's
 // phase, kept over the solves of a persistent launch; the barrier is
 // initialised by the caller.  Returns false when a bounded wait gave up.
-template <int DOT, int RPT, class S>
+template <int DOT, int RPT, int SLOTS, class S>
 __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t chunk, bool wide,
                                uint32_t smem_bytes, uint32_t& phase)
 {
     typedef DotT<DOT> D;
     typedef typename D::T T;
+    constexpr bool kLean = RPT > 2;
+    constexpr int G = RPT > 1 ? 2 : 4;
     const uint32_t n = c.n, B = blockDim.x, tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nw = B >> 5;
     const StepScalars* sc = c.sc;
     const uint32_t r0 = min(n, team.rank * chunk), r1 = min(n, r0 + chunk);
@@ -456,7 +465,7 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
     const uint32_t w0 = empty ? r0 : r0 > c.band ? r0 - c.band : 0u, w1 = empty ? r0 : min(n, r1 + c.band);
     const uint32_t W = res_window(n, chunk, c.band);
     float* P = reinterpret_cast<float*>(smem + kResHeader);
-    const bool zin = !S::kGrid && team.size > 1;
+    const bool zin = !S::kGrid && (kLean || team.size > 1);
     const uint32_t a_off = res_block_offset(n, chunk, c.band, zin, wide);
     uint16_t* list = reinterpret_cast<uint16_t*>(smem + kResHeader + 12u * W + (zin ? 12u * chunk : 0u));
     uint8_t* seen = reinterpret_cast<uint8_t*>(list + W);
@@ -471,12 +480,12 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
     }
     const uint32_t room = (smem_bytes - a_off) / 36u;  // blocks
 
-    // the resident slices: the first ones that fit
-    uint32_t qr = q1;
-    while (qr > q0 && c.slice_off[qr] - so0 > room) --qr;
+    // the resident slices: the first ones that fit (a CTA has fewer slices
+    // than threads); earlier reads of the buffer are done
+    const uint32_t qr =
+        q0 + (uint32_t)__syncthreads_count(q0 + tid < q1 && c.slice_off[q0 + tid + 1u] - so0 <= room);
     const bool copies = qr > q0;
     if (copies) {
-        __syncthreads();  // an earlier solve's reads of the buffer are done
         if (tid == 0) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&team.sh->mbar)),
@@ -496,16 +505,18 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
         }
     }
 
-    ResRow row[RPT];
-    f3 x[RPT], r[RPT], z[RPT], p[RPT], pv[RPT], s[RPT];
+    ResRow<SLOTS> row[RPT];
+    f3 r[RPT], s[RPT];
+    f3 x[kLean ? 1 : RPT], z[kLean ? 1 : RPT], p[kLean ? 1 : RPT], pv[kLean ? 1 : RPT];
     uint32_t flags = 0u;  // per row: bit i active, bit 8 + i dynamic, bit 16 + i resident
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
         const uint32_t q = q0 + warp + i * nw, g = 32u * q + lane;
-        row[i].off = row[i].cs = row[i].width = 0u;
-        x[i] = r[i] = z[i] = p[i] = s[i] = pv[i] = zero3();
+        row[i].off = row[i].width = 0u;
+        r[i] = s[i] = zero3();
+        if constexpr (!kLean) x[i] = z[i] = p[i] = pv[i] = zero3();
 #pragma unroll
-        for (int k = 0; k < kResSlots / 2; ++k) row[i].col[k] = 0u;
+        for (int k = 0; k < SLOTS / 2; ++k) row[i].col[k] = 0u;
         if (q < q1 && g < r1) {
             const uint32_t so = c.slice_off[q];
             const bool res = q < qr;
@@ -513,12 +524,11 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
             flags |= (1u << i) | (dyn ? 0x100u << i : 0u) | (res ? 0x10000u << i : 0u);
             const uint32_t len = c.slice_off[q + 1] - so;
             row[i].width = len >> 5;
-            row[i].cs = res ? len : c.E;
             row[i].off = (res ? 9u * (so - so0) : so) + lane;
 #pragma unroll
-            for (int k = 0; k < kResSlots; ++k)
+            for (int k = 0; k < SLOTS; ++k)
                 if ((uint32_t)k < row[i].width) row[i].col[k >> 1] |= (c.cols[so + lane + 32u * k] - w0) << ((k & 1) * 16);
-            pv[i] = ld3(c.pinv, n, g);
+            if constexpr (!kLean) pv[i] = ld3(c.pinv, n, g);
         }
     }
     const uint32_t below = r0 - w0;
@@ -530,7 +540,7 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
 #pragma unroll
         for (int i = 0; i < RPT; ++i)
 #pragma unroll
-            for (int k = 0; k < kResSlots; ++k)
+            for (int k = 0; k < SLOTS; ++k)
                 if ((uint32_t)k < row[i].width) seen[(k & 1) ? row[i].col[k >> 1] >> 16 : row[i].col[k >> 1] & 0xffffu] = 1;
         __syncthreads();
         for (uint32_t l = tid; l < w1 - w0; l += B)
@@ -604,16 +614,22 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
 #pragma unroll
             for (int i = 0; i < RPT; ++i)
                 if ((flags >> i) & 1u) {
-                    p[i] = first ? z[i] : z[i] + beta * p[i];
-                    stp(P, below + 32u * (warp + i * nw) + lane, p[i]);
+                    const uint32_t l = below + 32u * (warp + i * nw) + lane;
+                    if constexpr (kLean) {
+                        const f3 zi = ld3(team.zs, chunk, l - below);
+                        stp(P, l, first ? zi : zi + beta * ldp(P, l));
+                    } else {
+                        p[i] = first ? z[i] : z[i] + beta * p[i];
+                        stp(P, l, p[i]);
+                    }
                 }
             __syncthreads();
         }
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
             s[i] = zero3();
-            if ((flags >> (16 + i)) & 1u) s[i] = res_row_times(row[i], as_addr, P);
-            else if (row[i].width) s[i] = res_row_times(row[i], c.vals, P);
+            if ((flags >> (16 + i)) & 1u) s[i] = res_row_times<G>(row[i], as_addr, P);
+            else if (row[i].width) s[i] = res_row_times<2>(row[i], c.vals, c.E, P);
             if (!((flags >> (8 + i)) & 1u) && !start) s[i] = zero3();
         }
         if (start) {
@@ -626,14 +642,17 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
                     const uint32_t l = 32u * (warp + i * nw) + lane, g = r0 + l;
                     const bool dyn = (flags >> (8 + i)) & 1u;
                     const f3 bi = ld3(c.b, n, g);
-                    x[i] = ldp(P, g - w0);
+                    const f3 x0 = ldp(P, g - w0), pi = kLean ? ld3(c.pinv, n, g) : pv[kLean ? 0 : i];
+                    if constexpr (kLean) st3(c.dv, n, g, x0);
+                    else x[i] = x0;
                     r[i] = dyn ? bi - s[i] : zero3();
-                    z[i] = dyn ? mk(r[i].x * pv[i].x, r[i].y * pv[i].y, r[i].z * pv[i].z) : zero3();
-                    team.put_z(c, g, l, chunk, z[i]);
+                    const f3 zi = dyn ? mk(r[i].x * pi.x, r[i].y * pi.y, r[i].z * pi.z) : zero3();
+                    if constexpr (kLean) st3(team.zs, chunk, l, zi);
+                    else z[i] = zi, team.put_z(c, g, l, chunk, zi);
                     const f3 bh = dyn ? bi : zero3();
-                    const f3 w = c.cg_soft ? ld3(c.cg_diag, n, g) : pv[i];
+                    const f3 w = c.cg_soft ? ld3(c.cg_diag, n, g) : pi;
                     v2[0] = D::add_term(v2[0], bh, mk(bh.x * w.x, bh.y * w.y, bh.z * w.z));
-                    v2[1] = D::add_term(v2[1], r[i], z[i]);
+                    v2[1] = D::add_term(v2[1], r[i], zi);
                 }
             }
             // a copy that never landed ends the whole team's solve as a breakdown
@@ -655,7 +674,8 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
         T v1[1] = {D::zero()};
 #pragma unroll
         for (int i = 0; i < RPT; ++i)
-            if ((flags >> i) & 1u) v1[0] = D::add_term(v1[0], p[i], s[i]);
+            if ((flags >> i) & 1u)
+                v1[0] = D::add_term(v1[0], kLean ? ldp(P, below + 32u * (warp + i * nw) + lane) : p[kLean ? 0 : i], s[i]);
         if constexpr (S::kGrid) {
             team.template publish<D, 1>(v1);
             if (!team.template collect<D, 1>(v1)) return false;
@@ -670,11 +690,14 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
         for (int i = 0; i < RPT; ++i)
             if ((flags >> i) & 1u) {
                 const uint32_t l = 32u * (warp + i * nw) + lane;
-                x[i] = x[i] + alpha * p[i];
+                const f3 pi = kLean ? ld3(c.pinv, n, r0 + l) : pv[kLean ? 0 : i];
+                if constexpr (kLean) st3(c.dv, n, r0 + l, ld3(c.dv, n, r0 + l) + alpha * ldp(P, below + l));
+                else x[i] = x[i] + alpha * p[i];
                 r[i] = r[i] - alpha * s[i];
-                const f3 h = mk(r[i].x * pv[i].x, r[i].y * pv[i].y, r[i].z * pv[i].z);
-                z[i] = (flags >> (8 + i)) & 1u ? h : zero3();
-                team.put_z(c, r0 + l, l, chunk, z[i]);
+                const f3 h = mk(r[i].x * pi.x, r[i].y * pi.y, r[i].z * pi.z);
+                const f3 zi = (flags >> (8 + i)) & 1u ? h : zero3();
+                if constexpr (kLean) st3(team.zs, chunk, l, zi);
+                else z[i] = zi, team.put_z(c, r0 + l, l, chunk, zi);
                 u1[0] = D::add_term(u1[0], r[i], h);
             }
         if (!sum_and_halo(u1)) return false;
@@ -690,9 +713,11 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
         if (!isfinite(dn) || !isfinite(alpha) || !isfinite(beta)) status = kStatusNumerical;
         if (status != 0u || it >= max_iter || stop.met(dn)) break;
     }
+    if constexpr (!kLean) {
 #pragma unroll
-    for (int i = 0; i < RPT; ++i)
-        if ((flags >> i) & 1u) st3(c.dv, n, r0 + 32u * (warp + i * nw) + lane, x[i]);
+        for (int i = 0; i < RPT; ++i)
+            if ((flags >> i) & 1u) st3(c.dv, n, r0 + 32u * (warp + i * nw) + lane, x[i]);
+    }
     if (team.rank == 0 && tid == 0) {
         StepScalars* w = c.sc;
         w->b_delta = b_delta;

@@ -14,10 +14,13 @@ constexpr int kResMaxThreads = 512;
 constexpr int kResMaxTeam = 8;    // CTAs of a cluster
 constexpr int kResMaxGrid = 160;  // CTAs of a cooperative launch
 constexpr int kResSlots = 16;     // widest row
+constexpr int kResFewSlots = 8;   // widest row of the forms for few blocks a row
 constexpr int kResMaxWords = 128; // warps of a team
+constexpr int kResBatchRows = 4;  // most rows a thread in a batch
 constexpr int kResLine = 8;       // 16-byte words between two partials of a grid
 constexpr int kResHalo = 4;       // halo rows a thread
 constexpr uint32_t kResHeader = 4224;
+constexpr uint32_t kResBatchStatic = 2048;  // static shared memory of the batch's kernel
 constexpr uint32_t kResSmemLimit = 227 * 1024;
 
 // Rows whose direction a CTA of `chunk` rows keeps: its own and the band's.
@@ -33,6 +36,12 @@ __host__ __device__ inline uint32_t res_block_offset(uint32_t n, uint32_t chunk,
     const uint32_t b =
         kResHeader + (wide ? 15u : 12u) * res_window(n, chunk, band) + (z_in_smem ? 12u * chunk : 0u);
     return (b + 127u) & ~127u;
+}
+
+// Whether a CTA's halo is wider than its threads hold.
+__host__ __device__ inline bool res_wide(uint32_t n, uint32_t chunk, uint32_t band, uint32_t threads)
+{
+    return res_window(n, chunk, band) > (chunk < n ? chunk : n) + (uint32_t)kResHalo * threads;
 }
 
 struct ResShape {

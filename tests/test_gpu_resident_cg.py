@@ -61,3 +61,32 @@ def test_on_chip_cg_repeats_itself(b3g):
         cloth.step(scene.dt)
         runs.append(cloth.state()["dv"])
     assert all(np.array_equal(runs[0], r) for r in runs[1:])
+
+
+@pytest.mark.parametrize("cluster,split", [(1, ()), (8, tuple(range(32)))])
+@pytest.mark.parametrize("dot", [0, 2])
+def test_batch_on_chip_matches_launches(b3g, cluster, split, dot):
+    """Cloths at the edges of the batch's on-chip forms (one, two and four rows
+    a thread on one CTA and on a cluster, bending rows, a sewn pair, and one
+    past its reach): the same bound as above against each cloth stepped alone
+    with the per-iteration kernels or the on-chip CG."""
+    opts = b3g.SolverOptions(b3g.STOP_RELATIVE, 1e-9, 8, dot)
+    scenes = [b3g.plain_scene(2 if k == 0 else s) for k, s in enumerate((2, 22, 23, 32, 33, 45, 46, 64, 65, 91))]
+    scenes += [b3g.sphere_scene(22), b3g.sphere_scene(40), b3g.sewn_scene(20), b3g.plain_scene(130)]
+    small = b3g.SolverOptions(b3g.STOP_RELATIVE, 1e-9, 3, dot)
+    alone, cloths = [], []
+    for k, scene in enumerate(scenes):
+        rng = np.random.default_rng(k)
+        v = rng.normal(0.0, 0.1, (scene.mesh.vertex_count, 3)).astype(np.float32)
+        v[np.asarray(scene.pinned, np.int64)] = 0.0
+        for where in (alone, cloths):
+            c = b3g.Cloth(scene.mesh, scene.cdef).setup(scene, small if k == 0 else opts)
+            c.write_state(v=v, dv=0.1 * v)
+            where.append(c)
+    batch = b3g.Batch(len(cloths))
+    batch.set_schedule(cluster, split)
+    batch.step(cloths, scenes[0].dt)
+    for a, b in zip(alone, cloths):
+        a.step(scenes[0].dt)
+        x, y = a.state()["dv"].astype(np.float64), b.state()["dv"].astype(np.float64)
+        assert np.abs(x - y).max() <= (1e-6 if dot == 2 else 1e-5) * np.abs(x).max()
