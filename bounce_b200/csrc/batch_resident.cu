@@ -26,15 +26,15 @@ __device__ __forceinline__ void batch_solve(const ClothDev& c, TeamScope& team, 
 {
     const uint32_t slices = (c.n + 31u) >> 5, per = (slices + team.size - 1u) / team.size;
     const uint32_t chunk = 32u * per;
-    const bool wide = res_wide(c.n, chunk, c.band, blockDim.x);
     team.parity = 0u;
+    team.by_blocks = true;
     team.zs = reinterpret_cast<float*>(smem + kResHeader) + 3u * (size_t)res_window(c.n, chunk, c.band);
     if (per <= (uint32_t)kResMaxWarps)
-        resident_solve<DOT, 1, kResSlots>(c, team, smem, chunk, wide, smem_bytes, phase);
+        resident_solve<DOT, 1, kResSlots>(c, team, smem, chunk, 0u, smem_bytes, phase);
     else if (per <= 2u * kResMaxWarps)
-        resident_solve<DOT, 2, kResFewSlots>(c, team, smem, chunk, wide, smem_bytes, phase);
+        resident_solve<DOT, 2, kResFewSlots>(c, team, smem, chunk, 0u, smem_bytes, phase);
     else
-        resident_solve<DOT, kResBatchRows, kResFewSlots>(c, team, smem, chunk, wide, smem_bytes, phase);
+        resident_solve<DOT, kResBatchRows, kResFewSlots>(c, team, smem, chunk, 0u, smem_bytes, phase);
 }
 
 // A task is one cloth split over the cluster (count 0) or up to one cloth
@@ -102,9 +102,8 @@ bool batch_on_chip(const ClothDev& c, int team)
     const uint32_t slices = (c.n + 31u) / 32u, per = (slices + (uint32_t)team - 1u) / (uint32_t)team;
     if (per > (uint32_t)(kResBatchRows * kResMaxWarps)) return false;
     if (c.max_deg > (uint32_t)(per > (uint32_t)kResMaxWarps ? kResFewSlots : kResSlots)) return false;
-    const bool wide = res_wide(c.n, 32u * per, c.band, kResMaxThreads);
-    return (uint64_t)15u * res_window(c.n, 32u * per, c.band) <= kResSmemLimit / 2u &&
-           res_block_offset(c.n, 32u * per, c.band, true, wide) <= kResSmemLimit / 2u;
+    return !res_wide(c.n, 32u * per, c.band, kResMaxThreads) &&
+           res_block_offset(res_window(c.n, 32u * per, c.band), 12u * 32u * per) <= kResSmemLimit / 2u;
 }
 
 cudaError_t launch_batch_resident(const BatchCgArgs& a, int team, int dot, cudaStream_t st)

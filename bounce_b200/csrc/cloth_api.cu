@@ -140,7 +140,7 @@ b3g_status ensure_cg_rec(b3g_cloth* c)
 cudaError_t launch_persistent_cg(b3g_cloth* c, int dot, cudaStream_t st)
 {
     const ResShape shape = on_chip(c);
-    if (shape.ctas) return launch_resident_cg(c->dev, shape, dot, st);
+    if (shape.ctas) return launch_resident_cg(c->dev, shape, dot, c->cg_strategy == B3G_CG_LAUNCHES, st);
     cudaError_t e = cudaMemsetAsync(c->dev.bar, 0, kBarrierClear, st);
     if (e != cudaSuccess) return e;
     if (c->cg_strategy == B3G_CG_PERSISTENT_FUSED) return launch_grid_cg_fused(c->dev, dot, c->dev.bar, c->cg_rec, st);
@@ -376,6 +376,10 @@ b3g_status layout_cloth(b3g_cloth* c)
     d.max_deg = T.max_deg;
     d.band = T.band;
     d.E = T.E;
+    if (!c->lean_layout)  // (a server's cloths run in batches only)
+        resident_halos(d, [&](uint32_t i, auto&& f) {
+            for (uint32_t k = T.row_ptr[i]; k < T.row_ptr[i + 1]; ++k) f(T.row_cols[k]);
+        });
     d.k_stretch = def->streching;
     d.k_shear = def->shearing;
     d.k_damp = def->damping;
@@ -1835,7 +1839,7 @@ b3g_status b3g_debug_cg_barrier_timeout(b3g_cloth* c, uint32_t spin_limit, b3g_s
     } else {
         // (a cloth solved by one cluster waits on hardware barriers only)
         const ResShape shape = resident_shape(c->dev);
-        B3G_TRY(shape.ctas && shape.grid ? launch_resident_cg(c->dev, shape, (int)c->opts.dot, st)
+        B3G_TRY(shape.ctas && shape.grid ? launch_resident_cg(c->dev, shape, (int)c->opts.dot, false, st)
                                          : launch_grid_cg(c->dev, (int)c->opts.dot, c->dev.bar, st));
     }
     B3G_TRY(cudaMemsetAsync(c->dev.bar, 0, kBarrierReset, st));

@@ -89,6 +89,7 @@ struct ClothDev {
     uint32_t n, t, ns, nsph;
     uint32_t nslices, max_deg, E;
     uint32_t band;              // widest |row - column| of the matrix
+    uint32_t halo_team, halo_grid;  // resident_halos (resident_cg.h)
     const uint32_t* slice_off;  // nslices + 1
     const uint8_t* row_deg;     // n
     const uint32_t* cols;       // E

@@ -11,25 +11,27 @@ namespace {
 
 template <int DOT, int RPT, int SLOTS>
 __global__ void __launch_bounds__(kResMaxThreads, 1)
-    k_resident_team(const __grid_constant__ ClothDev c, uint32_t chunk, uint32_t wide, uint32_t smem_bytes)
+    k_resident_team(const __grid_constant__ ClothDev c, uint32_t chunk, uint32_t listed, uint32_t by_blocks,
+                    uint32_t smem_bytes)
 {
     extern __shared__ __align__(128) char smem[];
     ResShared* sh = reinterpret_cast<ResShared*>(smem);
     TeamScope team;
+    team.by_blocks = by_blocks != 0u;
     team.size = gridDim.x;  // one cluster
     team.rank = blockIdx.x;
     team.parity = 0u;
     team.sh = sh;
-    team.zs = reinterpret_cast<float*>(smem + kResHeader) + 3u * (size_t)res_window(c.n, chunk, c.band);
+    team.zs = reinterpret_cast<float*>(smem + kResHeader) + 3u * (size_t)res_rows(c.n, chunk, c.band, listed);
     uint32_t phase = 0u;
     res_init_copy_barrier(sh);
-    resident_solve<DOT, RPT, SLOTS>(c, team, smem, chunk, wide != 0u, smem_bytes, phase);
+    resident_solve<DOT, RPT, SLOTS>(c, team, smem, chunk, listed, smem_bytes, phase);
     team.barrier();  // no CTA leaves while another may still write into it
 }
 
 template <int DOT, int RPT, int SLOTS>
 __global__ void __launch_bounds__(kResMaxThreads, 1)
-    k_resident_grid(const __grid_constant__ ClothDev c, uint32_t chunk, uint32_t wide, uint32_t smem_bytes)
+    k_resident_grid(const __grid_constant__ ClothDev c, uint32_t chunk, uint32_t listed, uint32_t, uint32_t smem_bytes)
 {
     extern __shared__ __align__(128) char smem[];
     ResShared* sh = reinterpret_cast<ResShared*>(smem);
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1)
     team.arrivals = *(volatile uint32_t*)&c.bar->arrivals;
     uint32_t phase = 0u;
     res_init_copy_barrier(sh);
-    const bool good = resident_solve<DOT, RPT, SLOTS>(c, team, smem, chunk, wide != 0u, smem_bytes, phase);
+    const bool good = resident_solve<DOT, RPT, SLOTS>(c, team, smem, chunk, listed, smem_bytes, phase);
     if (threadIdx.x == 0 && !good) {
         c.sc->status = kResTimeout;
         c.sc->cont = 0;
@@ -66,41 +68,62 @@ const void* kernel_of(bool grid)
     return grid ? (const void*)k_resident_grid<DOT, RPT, SLOTS> : (const void*)k_resident_team<DOT, RPT, SLOTS>;
 }
 template <int DOT>
-const void* kernel_for(bool grid, uint32_t rpt, bool few)
+const void* kernel_for(bool grid, uint32_t rpt, uint32_t deg)
 {
-    if (rpt == 1) return kernel_of<DOT, 1, kResSlots>(grid);
-    return few ? kernel_of<DOT, 2, kResFewSlots>(grid) : kernel_of<DOT, 2, kResSlots>(grid);
+    if (rpt == 1)
+        return deg <= (uint32_t)kResSlots ? kernel_of<DOT, 1, kResSlots>(grid) : kernel_of<DOT, 1, kResWideSlots>(grid);
+    return deg <= (uint32_t)kResFewSlots ? kernel_of<DOT, 2, kResFewSlots>(grid) : kernel_of<DOT, 2, kResSlots>(grid);
 }
 
 }  // namespace
 
+uint32_t resident_team(uint32_t n)
+{
+    if (n > (uint32_t)(kResMaxTeam * kResMaxThreads)) return 0u;
+    uint32_t t = 1;
+    while (n > 256u && t < (uint32_t)kResMaxTeam && n > t * 128u) t *= 2;
+    return t;
+}
+
+uint32_t resident_chunk(uint32_t n, bool grid)
+{
+    const uint32_t slices = (n + 31u) / 32u, ctas = grid ? 148u : resident_team(n);
+    return ctas ? 32u * ((slices + ctas - 1u) / ctas) : 0u;
+}
+
 ResShape resident_shape(const ClothDev& c)
 {
     ResShape s;
-    if (c.max_deg > (uint32_t)kResSlots || c.n == 0) return s;
+    if (c.max_deg > (uint32_t)kResWideSlots || c.n == 0) return s;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const uint32_t n = c.n, slices = (n + 31u) / 32u;
     auto shape = [&](bool grid, uint32_t ctas) {
         ResShape r;
-        const uint32_t per = (slices + ctas - 1u) / ctas;
+        const uint32_t per = (slices + ctas - 1u) / ctas, most = (uint32_t)kResMaxThreads;
         r.grid = grid;
         r.chunk = 32u * per;
         r.ctas = grid ? (n + r.chunk - 1u) / r.chunk : ctas;
-        r.rows_per_thread = r.chunk <= (uint32_t)kResMaxThreads ? 1u : 2u;
-        r.threads = 32u * ((per + r.rows_per_thread - 1u) / r.rows_per_thread);
+        r.rows_per_thread = r.chunk <= most ? 1u : 2u;
+        const uint32_t own = 32u * ((per + r.rows_per_thread - 1u) / r.rows_per_thread);
         // threads without rows of their own help with the halo
-        const uint32_t halo = res_window(n, r.chunk, c.band) - std::min(n, r.chunk);
-        const uint32_t most = (uint32_t)kResMaxThreads;
-        r.threads = std::max(r.threads, std::min(most, 32u * ((halo + 32u * kResHalo - 1u) / (32u * kResHalo))));
+        const bool wide = res_wide(n, r.chunk, c.band, most);
+        if (wide && r.chunk == resident_chunk(n, grid)) r.listed = grid ? c.halo_grid : c.halo_team;
+        const uint32_t halo = wide ? r.listed : res_window(n, r.chunk, c.band) - std::min(n, r.chunk);
+        r.threads = std::max(own, 32u * ((halo + 32u * kResHalo - 1u) / (32u * kResHalo)));
         if (grid) r.threads = std::max(r.threads, 32u * ((r.ctas + 31u) / 32u));  // a thread a partial
-        r.wide = res_wide(n, r.chunk, c.band, r.threads);
-        const uint64_t off = res_block_offset(n, r.chunk, c.band, !grid && ctas > 1u, r.wide);
-        const uint64_t all = off + (uint64_t)r.chunk * c.max_deg * 36u;
+        const uint64_t off = res_block_offset(res_rows(n, r.chunk, c.band, r.listed),
+                                              !grid && ctas > 1u ? 12u * r.chunk : 0u);
+        // (listing needs two words a 32 rows and one a halo row beside the window)
+        const uint64_t all = off + std::max<uint64_t>((uint64_t)r.chunk * c.max_deg * 36u,
+                                            r.listed ? 8ull * slices + 4ull * r.listed : 0ull);
         r.smem = (uint32_t)std::min<uint64_t>(all, kResSmemLimit);
-        // at least half of the blocks resident
-        if (r.threads > most || off + (uint64_t)r.chunk * c.max_deg * 18u > kResSmemLimit) r.ctas = 0;
+        if ((wide && !r.listed) || r.threads > most) r.ctas = 0;
+        // at least half of the blocks resident, on average
+        if (off + (uint64_t)per * (c.E / slices) * 18u > kResSmemLimit) r.ctas = 0;
+        if (r.listed && off + 8ull * slices + 4ull * r.listed > kResSmemLimit) r.ctas = 0;
+        if (r.rows_per_thread > 1u && c.max_deg > (uint32_t)kResSlots) r.ctas = 0;
         return r;
     };
     // One CTA to 256 rows, then clusters of up to 8 CTAs of 128 to 512 rows,
@@ -108,21 +131,18 @@ ResShape resident_shape(const ClothDev& c)
     // rows 2.6 us on one CTA and 2.9 on two; 1,024 rows 3.3 on eight CTAs, 4.2
     // on two; 4,096 rows 4.5 on eight and 6.2 on the grid; 8,281 rows (13
     // blocks) 8.5 on a cluster of 16 and 5.4 on the grid.
-    uint32_t t = 1;
-    while (n > 256u && t < 8u && n > t * 128u) t *= 2;
-    if (n <= 8u * (uint32_t)kResMaxThreads) {
+    if (const uint32_t t = resident_team(n)) {
         s = shape(false, t);
         if (s.ctas) return s;
     }
     return shape(true, (uint32_t)std::min(sms, kResMaxGrid));
 }
 
-cudaError_t launch_resident_cg(const ClothDev& c, const ResShape& s, int dot, cudaStream_t st)
+cudaError_t launch_resident_cg(const ClothDev& c, const ResShape& s, int dot, bool by_blocks, cudaStream_t st)
 {
-    const bool few = c.max_deg <= (uint32_t)kResFewSlots;
-    const void* fn = dot == 2 ? kernel_for<2>(s.grid, s.rows_per_thread, few)
-                   : dot == 1 ? kernel_for<1>(s.grid, s.rows_per_thread, few)
-                              : kernel_for<0>(s.grid, s.rows_per_thread, few);
+    const void* fn = dot == 2 ? kernel_for<2>(s.grid, s.rows_per_thread, c.max_deg)
+                   : dot == 1 ? kernel_for<1>(s.grid, s.rows_per_thread, c.max_deg)
+                              : kernel_for<0>(s.grid, s.rows_per_thread, c.max_deg);
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemLimit);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
@@ -142,8 +162,8 @@ cudaError_t launch_resident_cg(const ClothDev& c, const ResShape& s, int dot, cu
     }
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    uint32_t chunk = s.chunk, wide = s.wide ? 1u : 0u, bytes = s.smem;
-    void* args[4] = {const_cast<ClothDev*>(&c), &chunk, &wide, &bytes};
+    uint32_t chunk = s.chunk, listed = s.listed, blocks = by_blocks ? 1u : 0u, bytes = s.smem;
+    void* args[5] = {const_cast<ClothDev*>(&c), &chunk, &listed, &blocks, &bytes};
     e = cudaLaunchKernelExC(&cfg, fn, args);
     count_launches(1);
     return e;

@@ -7,8 +7,9 @@
 //    component q is one contiguous run of 128 bytes a slot), as many slices as
 //    fit; the rest are read from L2 in every product;
 //  * the direction p of its window: its own rows and every row within `band`
-//    of them (band = the widest |row - column| of the matrix), so a product
-//    gathers p from shared memory only.
+//    of them (band = the widest |row - column| of the matrix) or, where few
+//    rows of so wide a band are needed, those it lists at the start; so a
+//    product gathers p from shared memory only.
 // x, r, z, p and P^-1 of its own rows and their column indices stay in
 // registers (with more than two rows a thread, x and P^-1 in L2, z in shared memory
 // and p in its window).  Per iteration only z of the window's halo crosses CTAs: the
@@ -53,7 +54,9 @@ struct ResShared {
     double wsum[2][2][kResMaxWords];  // [parity][value][warp of the team]
     unsigned long long mbar;
     int lost;
-    uint32_t listed;  // wide windows: halo rows the CTA's rows touch
+    uint32_t copied;               // blocks made resident
+    uint32_t len[kResMaxSlices];   // per slice of the CTA: its blocks,
+    uint32_t at[kResMaxSlices];    // and where they lie (~0: in L2)
 };
 static_assert(sizeof(ResShared) <= kResHeader, "fixed shared memory of the resident CG");
 
@@ -84,30 +87,39 @@ __device__ __forceinline__ typename D::T warp_sum(typename D::T v)
     return v;
 }
 
-// The sum of up to 16 8-byte words in shared memory by one thread, in the
-// order of block_reduce and grid_reduce (cg_common.cuh) over blocks of eight
-// warps: a tree over each eight, then the two.
+// The sum of `count` 8-byte words in shared memory, a warp's sum each, in the
+// order of the kernels these solves stand in for, so that FP32 sums come out
+// the same.  by_blocks: block_reduce and grid_reduce (cg_common.cuh) over
+// blocks of eight warps, a tree over each eight and a tree over the blocks;
+// else the cooperative CG's (grid_cg.cu) for one-warp CTAs: lane l adds words
+// l, l + 32, ... and a shuffle tree adds the lanes.  Up to 16 words by one
+// thread, else by a warp with the sum in lane 0.
 template <class D>
-__device__ __forceinline__ typename D::T words_sum(const double* w, uint32_t count)
+__device__ __forceinline__ typename D::T words_sum(const double* w, uint32_t count, bool by_blocks)
 {
     typedef typename D::T T;
     T a[kResMaxWarps];
 #pragma unroll
     for (uint32_t k = 0; k < (uint32_t)kResMaxWarps; ++k)
         a[k] = k < count ? *reinterpret_cast<const T*>(w + k) : D::zero();
+    if (by_blocks) {
 #pragma unroll
-    for (int step = 4; step > 0; step >>= 1)
+        for (int step = 4; step > 0; step >>= 1)
 #pragma unroll
-        for (int k = 0; k < step; ++k) {
-            a[k] = D::combine(a[k], a[k + step]);
-            a[k + 8] = D::combine(a[k + 8], a[k + 8 + step]);
-        }
-    return D::combine(a[0], a[8]);
+            for (int k = 0; k < step; ++k) {
+                a[k] = D::combine(a[k], a[k + step]);
+                a[k + 8] = D::combine(a[k + 8], a[k + 8 + step]);
+            }
+        return D::combine(a[0], a[8]);
+    }
+#pragma unroll
+    for (int step = kResMaxWarps / 2; step > 0; step >>= 1)
+#pragma unroll
+        for (int k = 0; k < step; ++k) a[k] = D::combine(a[k], a[k + step]);
+    return a[0];
 }
-
-// The same order for up to 128 words, by a warp: the sum in lane 0.
 template <class D>
-__device__ __forceinline__ typename D::T words_sum_warp(const double* w, uint32_t count)
+__device__ __forceinline__ typename D::T words_sum_warp(const double* w, uint32_t count, bool by_blocks)
 {
     typedef typename D::T T;
     const uint32_t lane = threadIdx.x & 31u;
@@ -116,9 +128,15 @@ __device__ __forceinline__ typename D::T words_sum_warp(const double* w, uint32_
     for (uint32_t m = 0; m < (uint32_t)kResMaxWords / 32u; ++m) {
         const uint32_t i = lane + 32u * m;
         a[m] = i < count ? *reinterpret_cast<const T*>(w + i) : D::zero();
-        if (32u * m < count)
+        if (by_blocks && 32u * m < count)
 #pragma unroll
             for (int off = 4; off > 0; off >>= 1) a[m] = D::combine(a[m], D::shfl(a[m], off));
+    }
+    if (!by_blocks) {
+#pragma unroll
+        for (uint32_t m = 1; m < (uint32_t)kResMaxWords / 32u; ++m)
+            if (lane + 32u * m < count) a[0] = D::combine(a[0], a[m]);
+        return warp_sum<D>(a[0]);
     }
     // blocks 4 m + lane / 8: a tree over sixteen
     if (count > 32u) {
@@ -135,6 +153,7 @@ struct TeamScope {
     static constexpr bool kGrid = false;
     uint32_t rank, size, parity;
     uint32_t word, words;  // this warp's word of the sums (kResMaxWords: none), and how many there are
+    bool by_blocks;        // the order of the sums (words_sum)
     ResShared* sh;
     float* zs;  // 3 planes of `chunk`: z of this CTA's rows, read by the team
 
@@ -167,8 +186,8 @@ struct TeamScope {
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             const double* w = sh->wsum[parity][k];
-            if (words <= (uint32_t)kResMaxWarps) v[k] = words_sum<D>(w, words);
-            else v[k] = unpack8<T>(__shfl_sync(0xffffffffu, pack8(words_sum_warp<D>(w, words)), 0));
+            if (words <= (uint32_t)kResMaxWarps) v[k] = words_sum<D>(w, words, by_blocks);
+            else v[k] = unpack8<T>(__shfl_sync(0xffffffffu, pack8(words_sum_warp<D>(w, words, by_blocks)), 0));
         }
         return true;
     }
@@ -228,11 +247,7 @@ struct GridScope {
         for (uint32_t spins = 0;; ++spins) {
             get(reinterpret_cast<const ulonglong2*>(zt + row), a, b);
             if ((uint32_t)(b >> 32) == tag) break;
-            if (spins > limit || ((spins & 63u) == 63u && failed())) {
-                sh->lost = 1;
-                fail();
-                break;
-            }
+            if (give_up(spins)) break;
         }
         return f3{__uint_as_float((uint32_t)a), __uint_as_float((uint32_t)(a >> 32)), __uint_as_float((uint32_t)b)};
     }
@@ -240,7 +255,7 @@ struct GridScope {
     // The grid's sums.  Each CTA counts itself in and publishes its partial as
     // one tagged 16-byte word in a line of its own; once the count is full,
     // thread r of every CTA reads rank r's partial, and all sum them in the
-    // same order (a shuffle tree a warp, then the warps in order).  Neither the
+    // same order (lane l ranks l, l + 32, ..., then a shuffle tree).  Neither the
     // count nor the partials carry a fence: a partial that is not there yet is
     // known by its tag and looked at again.  One thread a CTA polls the count
     // because polling all partials from every CTA delays the stores they wait
@@ -254,71 +269,68 @@ struct GridScope {
     {
         typedef typename D::T T;
         const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+        double* w = &sh->wsum[0][0][0];
         ++epoch;
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
             const T a = warp_sum<D>(v[k]);
-            if (lane == 0) *reinterpret_cast<T*>(&sh->wsum[0][k][warp]) = a;
+            if (lane == 0) *reinterpret_cast<T*>(w + k * kResMaxWarps + warp) = a;
         }
         __syncthreads();
         if (mute) return;
         if (threadIdx.x == 0)
             asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(&bar->arrived) : "memory");
-        if (threadIdx.x < (uint32_t)NV)
-            put(part + (((epoch & 1u) * 2u + lane) * kResMaxGrid + rank) * kResLine,
-                pack8(words_sum<D>(sh->wsum[0][lane], nw)), base + epoch);
+        if (threadIdx.x < (uint32_t)NV) {
+            // the warps in order, as the cooperative CG (grid_cg.cu) adds them
+            const double* mine = w + threadIdx.x * kResMaxWarps;
+            T a = *reinterpret_cast<const T*>(mine);
+            for (uint32_t q = 1; q < nw; ++q) a = D::combine(a, *reinterpret_cast<const T*>(mine + q));
+            put(part + (((epoch & 1u) * 2u + lane) * kResMaxGrid + rank) * kResLine, pack8(a), base + epoch);
+        }
+    }
+    __device__ bool give_up(uint32_t spins) const
+    {
+        if (spins <= limit && ((spins & 63u) != 63u || !failed())) return false;
+        sh->lost = 1;
+        fail();
+        return true;
     }
     template <class D, int NV>
     __device__ bool collect(typename D::T (&v)[NV])
     {
         typedef typename D::T T;
-        const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+        const uint32_t lane = threadIdx.x & 31u;
+        double* w = &sh->wsum[0][0][0] + 2 * kResMaxWarps;  // [value][rank]
         if (threadIdx.x == 0) {
             const uint32_t target = arrivals + epoch * size;
             for (uint32_t spins = 0;; ++spins) {
                 uint32_t a;
                 asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(a) : "l"(&bar->arrived) : "memory");
-                if ((int32_t)(a - target) >= 0) break;
-                if (spins > limit || ((spins & 63u) == 63u && failed())) {
-                    sh->lost = 1;
-                    fail();
-                    break;
-                }
+                if ((int32_t)(a - target) >= 0 || give_up(spins)) break;
             }
         }
         __syncthreads();
-        if (warp * 32u < size) {
-            const ulonglong2* buf = part + ((epoch & 1u) * 2u * kResMaxGrid + threadIdx.x) * kResLine;
-            const unsigned long long tag = base + epoch;
-            const bool mine = threadIdx.x < size;
+        if (threadIdx.x < size) {
+            const uint32_t r = threadIdx.x;
 #pragma unroll
             for (int k = 0; k < NV; ++k) {
-                T a = D::zero();
-                if (mine) {
-                    unsigned long long u, t;
-                    for (uint32_t spins = 0;; ++spins) {
-                        get(buf + k * kResMaxGrid * kResLine, u, t);
-                        if (t == tag) break;
-                        if (spins > limit || ((spins & 63u) == 63u && failed())) {
-                            sh->lost = 1;
-                            fail();
-                            break;
-                        }
-                    }
-                    a = unpack8<T>(u);
+                const ulonglong2* from = part + (((epoch & 1u) * 2u + k) * kResMaxGrid + r) * kResLine;
+                unsigned long long u, t;
+                for (uint32_t spins = 0;; ++spins) {
+                    get(from, u, t);
+                    if (t == base + epoch || give_up(spins)) break;
                 }
-                a = warp_sum<D>(a);
-                if (lane == 0) *reinterpret_cast<T*>(&sh->wsum[1][k][warp]) = a;
+                *reinterpret_cast<T*>(w + k * kResMaxGrid + r) = unpack8<T>(u);
             }
         }
         __syncthreads();
 #pragma unroll
         for (int k = 0; k < NV; ++k) {
-            T a = *reinterpret_cast<const T*>(&sh->wsum[1][k][0]);
+            T a = D::zero();
 #pragma unroll
-            for (uint32_t w = 1; w < (uint32_t)kResMaxGrid / 32u; ++w)
-                if (32u * w < size) a = D::combine(a, *reinterpret_cast<const T*>(&sh->wsum[1][k][w]));
-            v[k] = a;
+            for (uint32_t m = 0; m < (uint32_t)kResMaxGrid / 32u; ++m)
+                if (lane + 32u * m < size) a = D::combine(a, *reinterpret_cast<const T*>(w + k * kResMaxGrid + lane + 32u * m));
+            v[k] = unpack8<T>(__shfl_sync(0xffffffffu, pack8(warp_sum<D>(a)), 0));
         }
         return sh->lost == 0;
     }
@@ -444,14 +456,13 @@ __device__ __forceinline__ f3 res_row_times(const R& r, const float* blocks, uin
 }
 
 // The whole solve by a team.  `smem`: kResHeader bytes (the scope's
-// ResShared), then P (3 W floats), zs (3 chunk floats, clusters only), then
-// the blocks from a_off on, up to smem_bytes.  `wide`: most of the window is
-// not needed (few couplings reach far), so the CTA lists the halo rows that
-// its rows touch.  `phase`: the copy barrier's
+// ResShared), then P (3 floats a row of the window), zs (3 chunk floats, clusters only), then
+// the blocks from a_off on, up to smem_bytes.  `listed`: the CTA keeps p of the rows its rows touch
+// (c.halo of them at most) instead of the band's.  `phase`: the copy barrier's
 // phase, kept over the solves of a persistent launch; the barrier is
 // initialised by the caller.  Returns false when a bounded wait gave up.
 template <int DOT, int RPT, int SLOTS, class S>
-__device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t chunk, bool wide,
+__device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t chunk, uint32_t listed,
                                uint32_t smem_bytes, uint32_t& phase)
 {
     typedef DotT<DOT> D;
@@ -463,15 +474,13 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
     const uint32_t r0 = min(n, team.rank * chunk), r1 = min(n, r0 + chunk);
     const bool empty = r0 == r1;  // a CTA past the last row still joins the reductions
     const uint32_t w0 = empty ? r0 : r0 > c.band ? r0 - c.band : 0u, w1 = empty ? r0 : min(n, r1 + c.band);
-    const uint32_t W = res_window(n, chunk, c.band);
+    // Local numbering of p: by band, the window from w0 on; listed (most of the
+    // band is not needed), the CTA's rows and then the halo rows they touch.
     float* P = reinterpret_cast<float*>(smem + kResHeader);
     const bool zin = !S::kGrid && (kLean || team.size > 1);
-    const uint32_t a_off = res_block_offset(n, chunk, c.band, zin, wide);
-    uint16_t* list = reinterpret_cast<uint16_t*>(smem + kResHeader + 12u * W + (zin ? 12u * chunk : 0u));
-    uint8_t* seen = reinterpret_cast<uint8_t*>(list + W);
+    const uint32_t a_off = res_block_offset(res_rows(n, chunk, c.band, listed), zin ? 12u * chunk : 0u);
     float* As = reinterpret_cast<float*>(smem + a_off);
     const uint32_t q0 = r0 >> 5, q1 = empty ? q0 : (r1 + 31u) >> 5;
-    const uint32_t so0 = c.slice_off[q0];
     if constexpr (!S::kGrid) {
         // one row a thread: a word a slice, summed in the order of the
         // per-iteration kernels (their FP32 sums come out the same)
@@ -479,36 +488,82 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
         team.words = RPT > 1 ? team.size * nw : (n + 31u) >> 5;
     }
     const uint32_t room = (smem_bytes - a_off) / 36u;  // blocks
-
-    // the resident slices: the first ones that fit (a CTA has fewer slices
-    // than threads); earlier reads of the buffer are done
-    const uint32_t qr =
-        q0 + (uint32_t)__syncthreads_count(q0 + tid < q1 && c.slice_off[q0 + tid + 1u] - so0 <= room);
-    const bool copies = qr > q0;
-    if (copies) {
-        if (tid == 0) {
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&team.sh->mbar)),
-                         "r"((c.slice_off[qr] - so0) * 36u)
-                         : "memory");
+    // The resident slices: the widest that fit, since a slice left in L2 costs
+    // its row's loads in turn.  (A CTA has at most kResMaxSlices slices.)
+    __syncthreads();  // earlier reads of the buffer and of these are done
+    const uint32_t nq = q1 - q0;
+    if (tid < nq) team.sh->len[tid] = c.slice_off[q0 + tid + 1u] - c.slice_off[q0 + tid];
+    if (tid == 0) team.sh->copied = 0u;
+    __syncthreads();
+    if (tid < nq) {
+        const uint32_t len = team.sh->len[tid];
+        uint32_t before = 0u;
+        for (uint32_t j = 0; j < nq; ++j) {
+            const uint32_t o = team.sh->len[j];
+            if (o > len || (o == len && j < tid)) before += o;
         }
-        __syncthreads();
-        for (uint32_t k = tid; k < 9u * (qr - q0); k += B) {
-            const uint32_t q = q0 + k / 9u, comp = k % 9u;
-            const uint32_t so = c.slice_off[q], len = c.slice_off[q + 1] - so;
-            if (len)
-                asm volatile(
-                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                        smem_addr(As + 9u * (size_t)(so - so0) + (size_t)comp * len)),
-                    "l"(c.vals + (size_t)comp * c.E + so), "r"(len * 4u), "r"(smem_addr(&team.sh->mbar))
-                    : "memory");
-        }
+        const bool fits = before + len <= room;
+        team.sh->at[tid] = fits ? before : ~0u;
+        if (fits) atomicAdd(&team.sh->copied, len);
     }
+    __syncthreads();
 
     ResRow<SLOTS> row[RPT];
     f3 r[RPT], s[RPT];
     f3 x[kLean ? 1 : RPT], z[kLean ? 1 : RPT], p[kLean ? 1 : RPT], pv[kLean ? 1 : RPT];
     uint32_t flags = 0u;  // per row: bit i active, bit 8 + i dynamic, bit 16 + i resident
+    const uint32_t below = listed ? 0u : r0 - w0;  // local index of the CTA's first row
+    uint32_t halo = r0 - w0 + (w1 - r1);
+    uint32_t* bits = reinterpret_cast<uint32_t*>(As);  // scratch until the blocks are copied: a bit a row,
+    uint32_t* rank_of = bits + (n + 31u) / 32u;        // the bits before each word,
+    uint32_t* rows_of = rank_of + (n + 31u) / 32u;     // and the listed rows
+    if (listed) {
+        const uint32_t words = (n + 31u) / 32u;
+        for (uint32_t i = tid; i < words; i += B) bits[i] = 0u;
+        __syncthreads();
+        for (uint32_t q = q0 + warp; q < q1; q += nw)
+            for (uint32_t o = c.slice_off[q] + lane; o < c.slice_off[q + 1]; o += 32u) {
+                const uint32_t col = c.cols[o];
+                if (col < r0 || col >= r1) atomicOr(bits + (col >> 5), 1u << (col & 31u));
+            }
+        __syncthreads();
+        // thread t numbers the rows of its run of words
+        const uint32_t run = (words + B - 1u) / B, i0 = min(words, tid * run), i1 = min(words, i0 + run);
+        uint32_t mine = 0u;
+        for (uint32_t i = i0; i < i1; ++i) mine += __popc(bits[i]);
+        uint32_t upto = mine;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, upto, off);
+            if (lane >= (uint32_t)off) upto += o;
+        }
+        uint32_t* warp_total = reinterpret_cast<uint32_t*>(&team.sh->wsum[0][0][0]);
+        if (lane == 31u) warp_total[warp] = upto;
+        __syncthreads();
+        uint32_t at = upto - mine;
+        halo = 0u;
+        for (uint32_t q = 0; q < nw; ++q) {
+            if (q < warp) at += warp_total[q];
+            halo += warp_total[q];
+        }
+        for (uint32_t i = i0; i < i1; ++i) {
+            rank_of[i] = at;
+            for (uint32_t m = bits[i]; m; m &= m - 1u) rows_of[at++] = 32u * i + (uint32_t)__ffs(m) - 1u;
+        }
+        __syncthreads();
+    }
+    uint32_t hrow[kResHalo];  // the thread's halo rows
+#pragma unroll
+    for (int u = 0; u < kResHalo; ++u) {
+        const uint32_t h = tid + u * B;
+        hrow[u] = h >= halo ? ~0u : listed ? rows_of[h] : h < below ? w0 + h : r1 + (h - below);
+    }
+    auto halo_at = [&](int u) -> uint32_t { return listed ? chunk + tid + u * B : hrow[u] - w0; };
+    auto local = [&](uint32_t col) -> uint32_t {
+        if (!listed) return col - w0;
+        if (col >= r0 && col < r1) return col - r0;
+        return chunk + rank_of[col >> 5] + __popc(bits[col >> 5] & ((1u << (col & 31u)) - 1u));
+    };
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
         const uint32_t q = q0 + warp + i * nw, g = 32u * q + lane;
@@ -519,40 +574,47 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
         for (int k = 0; k < SLOTS / 2; ++k) row[i].col[k] = 0u;
         if (q < q1 && g < r1) {
             const uint32_t so = c.slice_off[q];
-            const bool res = q < qr;
+            const uint32_t at = team.sh->at[q - q0];
+            const bool res = at != ~0u;
             const bool dyn = c.type[g] == 2;
             flags |= (1u << i) | (dyn ? 0x100u << i : 0u) | (res ? 0x10000u << i : 0u);
             const uint32_t len = c.slice_off[q + 1] - so;
             row[i].width = len >> 5;
-            row[i].off = (res ? 9u * (so - so0) : so) + lane;
+            row[i].off = (res ? 9u * at : so) + lane;
 #pragma unroll
             for (int k = 0; k < SLOTS; ++k)
-                if ((uint32_t)k < row[i].width) row[i].col[k >> 1] |= (c.cols[so + lane + 32u * k] - w0) << ((k & 1) * 16);
+                if ((uint32_t)k < row[i].width)
+                    row[i].col[k >> 1] |= local(c.cols[so + lane + 32u * k]) << ((k & 1) * 16);
             if constexpr (!kLean) pv[i] = ld3(c.pinv, n, g);
         }
     }
-    const uint32_t below = r0 - w0;
-    uint32_t halo = below + (w1 - r1);
-    if (wide) {
-        for (uint32_t l = tid; l < W; l += B) seen[l] = 0;
-        if (tid == 0) team.sh->listed = 0u;
+    const bool copies = team.sh->copied != 0u;
+    if (copies) {
+        __syncthreads();  // the scratch is free
+        if (tid == 0) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&team.sh->mbar)),
+                         "r"(team.sh->copied * 36u)
+                         : "memory");
+        }
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < RPT; ++i)
-#pragma unroll
-            for (int k = 0; k < SLOTS; ++k)
-                if ((uint32_t)k < row[i].width) seen[(k & 1) ? row[i].col[k >> 1] >> 16 : row[i].col[k >> 1] & 0xffffu] = 1;
-        __syncthreads();
-        for (uint32_t l = tid; l < w1 - w0; l += B)
-            if (seen[l] && (l < below || l >= r1 - w0)) list[atomicAdd(&team.sh->listed, 1u)] = (uint16_t)l;
-        __syncthreads();
-        halo = team.sh->listed;
+        for (uint32_t k = tid; k < 9u * nq; k += B) {
+            const uint32_t q = k / 9u, comp = k % 9u;
+            const uint32_t at = team.sh->at[q], len = team.sh->len[q];
+            if (at != ~0u && len)
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                        smem_addr(As + 9u * (size_t)at + (size_t)comp * len)),
+                    "l"(c.vals + (size_t)comp * c.E + c.slice_off[q0 + q]), "r"(len * 4u), "r"(smem_addr(&team.sh->mbar))
+                    : "memory");
+        }
     }
-    // the window index of halo row h
-    auto halo_at = [&](uint32_t h) -> uint32_t { return wide ? list[h] : h < below ? h : r1 - w0 + (h - below); };
-    // x0 = S m_x over the window (cg_soft: on every row)
-    for (uint32_t j = w0 + tid; j < w1; j += B)
-        stp(P, j - w0, (c.cg_soft || c.type[j] == 2) ? ld3(c.mx, n, j) : zero3());
+    // x0 = S m_x over the CTA's rows and its halo (cg_soft: on every row)
+    auto start_at = [&](uint32_t j) -> f3 { return (c.cg_soft || c.type[j] == 2) ? ld3(c.mx, n, j) : zero3(); };
+    for (uint32_t j = r0 + tid; j < r1; j += B) stp(P, below + j - r0, start_at(j));
+#pragma unroll
+    for (int u = 0; u < kResHalo; ++u)
+        if (hrow[u] != ~0u) stp(P, halo_at(u), start_at(hrow[u]));
     bool landed = true;
     if (copies) {
         const uint32_t mb = smem_addr(&team.sh->mbar);
@@ -568,7 +630,7 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
     __syncthreads();
 
     const uint32_t as_addr = smem_addr(As);
-    f3 zh[kResHalo];  // z of the thread's first halo rows
+    f3 zh[kResHalo];  // z of the thread's halo rows
     uint32_t tag = 0u;
     // the sums of the phase that made z, and the halo's z
     auto sum_and_halo = [&](auto& v) -> bool {
@@ -582,10 +644,8 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
             good = team.template sum<D, NV>(v);
         }
 #pragma unroll
-        for (int u = 0; u < kResHalo; ++u) {
-            const uint32_t h = tid + u * B;
-            if (h < halo) zh[u] = team.get_z(c, w0 + halo_at(h), chunk, tag);
-        }
+        for (int u = 0; u < kResHalo; ++u)
+            if (hrow[u] != ~0u) zh[u] = team.get_z(c, hrow[u], chunk, tag);
         return good;
     };
     const uint32_t max_iter = sc->max_iter;
@@ -599,18 +659,11 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
             // the window's p = z + beta p_old (cloth_force_solver.cpp:130)
             const bool first = it == 0;
 #pragma unroll
-            for (int u = 0; u < kResHalo; ++u) {
-                const uint32_t h = tid + u * B;
-                if (h < halo) {
-                    const uint32_t l = halo_at(h);
+            for (int u = 0; u < kResHalo; ++u)
+                if (hrow[u] != ~0u) {
+                    const uint32_t l = halo_at(u);
                     stp(P, l, first ? zh[u] : zh[u] + beta * ldp(P, l));
                 }
-            }
-            for (uint32_t h = tid + kResHalo * B; h < halo; h += B) {
-                const uint32_t l = halo_at(h);
-                const f3 zj = team.get_z(c, w0 + l, chunk, tag);
-                stp(P, l, first ? zj : zj + beta * ldp(P, l));
-            }
 #pragma unroll
             for (int i = 0; i < RPT; ++i)
                 if ((flags >> i) & 1u) {
@@ -629,7 +682,7 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
         for (int i = 0; i < RPT; ++i) {
             s[i] = zero3();
             if ((flags >> (16 + i)) & 1u) s[i] = res_row_times<G>(row[i], as_addr, P);
-            else if (row[i].width) s[i] = res_row_times<2>(row[i], c.vals, c.E, P);
+            else if (row[i].width) s[i] = res_row_times<G>(row[i], c.vals, c.E, P);
             if (!((flags >> (8 + i)) & 1u) && !start) s[i] = zero3();
         }
         if (start) {
@@ -642,7 +695,7 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
                     const uint32_t l = 32u * (warp + i * nw) + lane, g = r0 + l;
                     const bool dyn = (flags >> (8 + i)) & 1u;
                     const f3 bi = ld3(c.b, n, g);
-                    const f3 x0 = ldp(P, g - w0), pi = kLean ? ld3(c.pinv, n, g) : pv[kLean ? 0 : i];
+                    const f3 x0 = ldp(P, below + l), pi = kLean ? ld3(c.pinv, n, g) : pv[kLean ? 0 : i];
                     if constexpr (kLean) st3(c.dv, n, g, x0);
                     else x[i] = x0;
                     r[i] = dyn ? bi - s[i] : zero3();

@@ -29,6 +29,7 @@
 #include "cloth_dev.cuh"
 #include "grid_cg.cuh"
 #include "mpcg_solve.cuh"
+#include "resident_cg.h"
 #include "hull_gjk.cuh"
 #include "softbody_prep.h"
 #include "vec.cuh"
@@ -774,6 +775,7 @@ b3g_status ensure_sell(b3g_softbody* b)
     }
     const uint32_t E = off[nslices];
     std::vector<uint32_t> cols(E);
+    uint32_t band = 0;
     for (uint32_t r = 0; r < n; ++r) {
         const uint32_t i = perm[r];
         const uint32_t width = (off[r / 32 + 1] - off[r / 32]) / 32;  // the slice's widest row
@@ -781,7 +783,9 @@ b3g_status ensure_sell(b3g_softbody* b)
         for (uint32_t k = 0; k < width; ++k) cols[off[r / 32] + 32 * k + (r & 31)] = r;  // padding
         for (uint32_t k = 0; k < deg[r]; ++k) {
             const uint32_t ss = k == dg ? 0u : k < dg ? k + 1u : k;  // the diagonal block first
-            cols[off[r / 32] + 32 * ss + (r & 31)] = inv[b->cols[b->rowptr[i] + k]];
+            const uint32_t col = inv[b->cols[b->rowptr[i] + k]];
+            cols[off[r / 32] + 32 * ss + (r & 31)] = col;
+            band = std::max(band, col > r ? col - r : r - col);
         }
     }
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
@@ -813,6 +817,8 @@ b3g_status ensure_sell(b3g_softbody* b)
     SB_TRY(cudaMemcpyAsync(d_deg, deg.data(), n, cudaMemcpyHostToDevice, s));
     SB_TRY(cudaMemcpyAsync(d_cols, cols.data(), (size_t)E * 4, cudaMemcpyHostToDevice, s));
     SB_TRY(cudaMemsetAsync(d_vals, 0, (size_t)E * 36, s));
+    SB_TRY(cudaMemsetAsync(partials, 0, kGridCgPartialBytes, s));
+    SB_TRY(cudaMemsetAsync(bar, 0, sizeof(GridBarrier), s));
     SB_TRY(cudaStreamSynchronize(s));  // the host vectors go out of scope
     SoftDev& d = b->dev;
     d.sell_vals = d_vals;
@@ -830,6 +836,7 @@ b3g_status ensure_sell(b3g_softbody* b)
     v.nslices = nslices;
     v.max_deg = max_deg;
     v.E = E;
+    v.band = band;
     v.slice_off = d_off;
     v.row_deg = d_deg;
     v.cols = d_cols;
@@ -847,14 +854,20 @@ b3g_status ensure_sell(b3g_softbody* b)
     v.type = d_type;
     v.sc = b->cs.sc;
     v.partials = partials;
+    v.bar = bar;
     v.cg_soft = 1;
+    resident_halos(v, [&](uint32_t r, auto&& f) {
+        for (uint32_t k = 0; k < deg[r]; ++k) f(cols[off[r / 32] + 32 * k + (r & 31)]);
+    });
     b->bar = bar;
     return B3G_OK;
 }
 
 // The soft body's MPCG (softbody_force_solver.cpp:93-164) as the cloth's
-// persistent cooperative CG in its soft body mode, on the SELL copy of the
-// system the assembly just wrote.
+// CG in its soft body mode, on the SELL copy of the system the assembly just
+// wrote: on chip where it fits (steps of blocks of 512, 9,261 and 68,921
+// nodes 150, 253 and 692 us, from 319, 386 and 817 with the cooperative CG
+// that reads the system from L2), else the cooperative launch.
 b3g_status persistent_cg(b3g_softbody* b, cudaStream_t s, StepScalars* h)
 {
     const ClothDev& v = b->view;
@@ -865,14 +878,18 @@ b3g_status persistent_cg(b3g_softbody* b, cudaStream_t s, StepScalars* h)
     init.tol = b->opts.tolerance;
     init.dot = (int)b->opts.dot;
     SB_TRY(cudaMemcpyAsync(v.sc, &init, sizeof(init), cudaMemcpyHostToDevice, s));
-    SB_TRY(cudaMemsetAsync(b->bar, 0, kBarrierClear, s));
-    SB_TRY(b->fused ? launch_grid_cg_fused(v, (int)b->opts.dot, b->bar, b->rec, s)
+    const ResShape shape = resident_shape(v);
+    if (!shape.ctas) SB_TRY(cudaMemsetAsync(b->bar, 0, kBarrierClear, s));
+    SB_TRY(shape.ctas ? launch_resident_cg(v, shape, (int)b->opts.dot, false, s)
+           : b->fused ? launch_grid_cg_fused(v, (int)b->opts.dot, b->bar, b->rec, s)
                     : launch_grid_cg(v, (int)b->opts.dot, b->bar, s));
     k_sb_from_planes<<<blocks_for(v.n), kBlock, 0, s>>>(v.dv, b->dev.sell_inv, b->cs.x, v.n);
     count_launches(1);
     SB_TRY(cudaGetLastError());
     SB_TRY(cudaMemcpyAsync(h, v.sc, sizeof(StepScalars), cudaMemcpyDeviceToHost, s));
     SB_TRY(cudaStreamSynchronize(s));
+    // a wait that gave up leaves the barrier's counts short
+    if (h->status == (uint32_t)B3G_ERR_TIMEOUT) SB_TRY(cudaMemsetAsync(b->bar, 0, kBarrierReset, s));
     return B3G_OK;
 }
 
