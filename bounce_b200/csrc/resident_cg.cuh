@@ -682,7 +682,7 @@ __device__ bool resident_solve(const ClothDev& c, S& team, char* smem, uint32_t 
         for (int i = 0; i < RPT; ++i) {
             s[i] = zero3();
             if ((flags >> (16 + i)) & 1u) s[i] = res_row_times<G>(row[i], as_addr, P);
-            else if (row[i].width) s[i] = res_row_times<G>(row[i], c.vals, c.E, P);
+            else if (row[i].width) s[i] = res_row_times<SLOTS == kResFewSlots ? 4 : G>(row[i], c.vals, c.E, P);
             if (!((flags >> (8 + i)) & 1u) && !start) s[i] = zero3();
         }
         if (start) {

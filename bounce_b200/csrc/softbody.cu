@@ -865,9 +865,12 @@ b3g_status ensure_sell(b3g_softbody* b)
 
 // The soft body's MPCG (softbody_force_solver.cpp:93-164) as the cloth's
 // CG in its soft body mode, on the SELL copy of the system the assembly just
-// wrote: on chip where it fits (steps of blocks of 512, 9,261 and 68,921
-// nodes 150, 253 and 692 us, from 319, 386 and 817 with the cooperative CG
-// that reads the system from L2), else the cooperative launch.
+// wrote: on chip where it fits (a step of blocks of 512, 9,261 and 28,768
+// nodes 149, 242 and 406 us, from 319, 386 and 535 with the cooperative CG
+// that reads the system from L2), else the cooperative launch.  The rows stay
+// in the order of their degree, which fixes the order of the FP32 sums; in
+// that order a CTA of a block of 68,921 nodes touches up to 2,817 rows
+// outside its own, more than its threads hold.
 b3g_status persistent_cg(b3g_softbody* b, cudaStream_t s, StepScalars* h)
 {
     const ClothDev& v = b->view;
