@@ -6,7 +6,7 @@
 //                   (softbody_force_solver.cpp:53-91), the element's f0 terms
 //                   R Ke x0 and its plastic strain update and plastic forces
 //                   (:256-357)
-//   k_sb_assemble   one warp per node: the node's row of K summed over its
+//   k_sb_assemble   8 to 32 lanes per node: the node's row of K summed over its
 //                   elements in element order (the reference's K(vi, vj) +=
 //                   R Ke RT), then b = M v - h (K p + f0 - (f_plastic + f_ext))
 //                   and A = M + h C + h^2 K (:359-377) in the reference's
@@ -18,8 +18,9 @@
 //
 // Node vectors are xyz per node (b3DenseVec3 layout).  With -fmad=false the
 // element and assembly arithmetic is the reference's; the one difference is
-// the C library's double sin and cos in b3Quat::Set against CUDA's, which can
-// differ in the last bit of the rounded float in rare cases.
+// the C library's double sin and cos in b3Quat::Set against the series and
+// CUDA's functions here, which can differ in the last bit of the rounded float
+// in rare cases.
 #include <algorithm>
 #include <cstring>
 #include <new>
@@ -44,14 +45,18 @@ struct SoftDev {
     float* damping;
     uint8_t* type;
     const uint4* tets;
-    const float *Ke, *invE, *B, *P;
+    const float4* shape;   // 3 per element (softbody_prep.h)
+    float lambda, mu, lambda2mu;
     float4* q;
     float* eps;
-    float *R, *f0s, *fps;
+    float4* R;             // 3 per element: the rotation's 9 floats, column-major
+    float *f0s, *fps;
     float c_yield, c_creep, c_max;
     const uint32_t *rowptr, *cols, *diag;
     float* vals;
     const uint32_t *inc_ptr, *inc_elem, *inc_meta;
+    const uint32_t* asm_nodes;  // the nodes by the lanes the assembly gives them: 32, 16, 8
+    uint32_t asm_count[3];
     float *b, *S, *xsol;
     float gx, gy, gz;
 
@@ -128,8 +133,27 @@ __device__ __forceinline__ float4 quat_mul(float4 a, float4 b)
                        a.w * b.z + a.z * b.w + a.x * b.y - a.y * b.x, a.w * b.w - a.x * b.x - a.y * b.y - a.z * b.z);
 }
 
+// sin and cos of a small angle in FP64 by their Taylor series: to 0.5 the first
+// term left out is below 2^-60 of the sum, so that the floats they are rounded
+// to are those of any correctly working sin and cos but for ties.
+__device__ __forceinline__ void small_sincos(double t, float& sine, float& cosine)
+{
+    const double u = t * t;
+    double s = -1.0 / 1307674368000.0, c = 1.0 / 20922789888000.0;
+    s = fma(s, u, 1.0 / 6227020800.0), c = fma(c, u, -1.0 / 87178291200.0);
+    s = fma(s, u, -1.0 / 39916800.0), c = fma(c, u, 1.0 / 479001600.0);
+    s = fma(s, u, 1.0 / 362880.0), c = fma(c, u, -1.0 / 3628800.0);
+    s = fma(s, u, -1.0 / 5040.0), c = fma(c, u, 1.0 / 40320.0);
+    s = fma(s, u, 1.0 / 120.0), c = fma(c, u, -1.0 / 720.0);
+    s = fma(s, u, -1.0 / 6.0), c = fma(c, u, 1.0 / 24.0);
+    c = fma(c, u, -0.5);
+    sine = (float)fma(s * u, t, t);
+    cosine = (float)fma(c, u, 1.0);
+}
+
 // b3ExtractRotation (softbody_force_solver.cpp:53-91): at most 20 steps of
-// the rotation update from the previous rotation q
+// the rotation update from the previous rotation q.  In FP32 the angle settles
+// near 1e-8 and seldom passes the stop, so an element usually runs all 20.
 __device__ m3 extract_rotation(float4& q, const m3& A)
 {
     for (int iteration = 0; iteration < 20; ++iteration) {
@@ -143,8 +167,14 @@ __device__ m3 extract_rotation(float4& q, const m3& A)
         if (w < 1.0e-9f) break;
         const f3 axis = omega / w;
         const float theta = 0.5f * w;
-        const float sine = (float)sin((double)theta);
-        const float4 oq = make_float4(sine * axis.x, sine * axis.y, sine * axis.z, (float)cos((double)theta));
+        float sine, cosine;
+        if (theta <= 0.5f) {
+            small_sincos((double)theta, sine, cosine);
+        } else {
+            sine = (float)sin((double)theta);
+            cosine = (float)cos((double)theta);
+        }
+        const float4 oq = make_float4(sine * axis.x, sine * axis.y, sine * axis.z, cosine);
         q = quat_mul(oq, q);
         const float len = sqrtf(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w);
         if (len > 1.1920929e-07f) {
@@ -165,7 +195,57 @@ __device__ __forceinline__ float len6(const float* v)
     return sqrtf(r);
 }
 
-__global__ void k_sb_elements(SoftDev d, float h, float inv_h)
+// The element matrices from the inverse edge matrix, the volume and the
+// material (softbody.cpp:43-155, :522-553): 48 bytes an element instead of
+// the 1,152 of Ke, B and P, and each entry the float that the reference's
+// matrix products give.  An entry of B^T D B sums over six strains in order,
+// and all but two or three of its terms are products with a zero of B or D,
+// which add nothing.
+struct Shape {
+    f3 g[4];   // rows of B: (b, c, d) of each vertex
+    float vol;
+};
+__device__ __forceinline__ m3 load_shape(const float4* s, Shape& q)
+{
+    const float4 a = __ldg(s), b = __ldg(s + 1), c = __ldg(s + 2);
+    q.g[0] = mk((a.x + a.y) + a.z, (a.w + b.x) + b.y, (b.z + b.w) + c.x);
+    q.g[1] = mk(-a.x, -a.w, -b.z);
+    q.g[2] = mk(-a.y, -b.x, -b.w);
+    q.g[3] = mk(-a.z, -b.y, -c.x);
+    q.vol = c.y;
+    return m3{f3{a.x, a.y, a.z}, f3{a.w, b.x, b.y}, f3{b.z, b.w, c.x}};  // invE
+}
+// Block (i, j), i <= j, of Ke = V B^T D B from the vertices' rows of B.
+__device__ __forceinline__ m3 stiffness_block(const SoftDev& d, f3 u, f3 v, float vol)
+{
+    const float L = d.lambda, M = d.mu, T = d.lambda2mu;
+    const float bT = u.x * T, bL = u.x * L, bM = u.x * M;
+    const float cT = u.y * T, cL = u.y * L, cM = u.y * M;
+    const float dT = u.z * T, dL = u.z * L, dM = u.z * M;
+    m3 k;
+    k.x.x = ((0.0f + bT * v.x) + cM * v.y) + dM * v.z;
+    k.x.y = (0.0f + cL * v.x) + bM * v.y;
+    k.x.z = (0.0f + dL * v.x) + bM * v.z;
+    k.y.x = (0.0f + bL * v.y) + cM * v.x;
+    k.y.y = ((0.0f + cT * v.y) + bM * v.x) + dM * v.z;
+    k.y.z = (0.0f + dL * v.y) + cM * v.z;
+    k.z.x = (0.0f + bL * v.z) + dM * v.x;
+    k.z.y = (0.0f + cL * v.z) + dM * v.y;
+    k.z.z = ((0.0f + dT * v.z) + bM * v.x) + cM * v.y;
+    return m3{f3{k.x.x * vol, k.x.y * vol, k.x.z * vol}, f3{k.y.x * vol, k.y.y * vol, k.y.z * vol},
+              f3{k.z.x * vol, k.z.y * vol, k.z.z * vol}};
+}
+__device__ __forceinline__ m3 load_rotation(const float4* r)
+{
+    const float4 a = r[0], b = r[1], c = r[2];
+    return m3{f3{a.x, a.y, a.z}, f3{a.w, b.x, b.y}, f3{b.z, b.w, c.x}};
+}
+
+// One thread per element: rotation, f0 terms, plastic strain and forces.
+// Bound: the rotation's double sine and cosine and about 2,500 float
+// operations an element; 364 bytes an element move (a 40^3 block: 96 us, of which
+// the bytes would take 18; 150 with the matrices read and CUDA's sin and cos).
+__global__ void __launch_bounds__(128) k_sb_elements(SoftDev d, float h, float inv_h)
 {
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= d.t) return;
@@ -177,55 +257,47 @@ __global__ void k_sb_elements(SoftDev d, float h, float inv_h)
         ps[k] = ldv(d.x, vs[k]);
         xs[k] = ldv(d.rest, vs[k]);
     }
+    Shape sh;
+    const m3 invE = load_shape(d.shape + 3 * (size_t)e, sh);
     const m3 E = m3{ps[1] - ps[0], ps[2] - ps[0], ps[3] - ps[0]};
-    const m3 A = mmul(E, ldm(d.invE + 9 * (size_t)e));
+    const m3 A = mmul(E, invE);
     float4 q = d.q[e];
     const m3 R = extract_rotation(q, A);
     d.q[e] = q;
     const m3 RT = transpose(R);
-    stm(d.R + 9 * (size_t)e, R);
-    // f0 terms: sum_j (R Ke_ij) x0_j.  Ke is read in memory order, 16 bytes
-    // per load: block (i, j) sits at 9 (i + 4 j), so the four blocks of one j
-    // are 36 consecutive floats; each of the four sums still runs over j in
-    // order.
-    const float4* Ke4 = reinterpret_cast<const float4*>(d.Ke + 144 * (size_t)e);
+    float4* Re = d.R + 3 * (size_t)e;
+    Re[0] = make_float4(R.x.x, R.x.y, R.x.z, R.y.x);
+    Re[1] = make_float4(R.y.y, R.y.z, R.z.x, R.z.y);
+    Re[2] = make_float4(R.z.z, 0.0f, 0.0f, 0.0f);
+    // f0 terms: sum_j (R Ke_ij) x0_j, over j in order; a block below the
+    // diagonal is the transpose of the one above it
     f3 f0acc[4] = {zero3(), zero3(), zero3(), zero3()};
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        float kb[36];
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            const float4 t4 = Ke4[9 * j + q];
-            kb[4 * q] = t4.x, kb[4 * q + 1] = t4.y, kb[4 * q + 2] = t4.z, kb[4 * q + 3] = t4.w;
+        for (int i = 0; i < 4; ++i) {
+            const m3 K = i <= j ? stiffness_block(d, sh.g[i], sh.g[j], sh.vol)
+                                : transpose(stiffness_block(d, sh.g[j], sh.g[i], sh.vol));
+            f0acc[i] = f0acc[i] + mmul(R, K) * xs[j];
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) f0acc[i] = f0acc[i] + mmul(R, ldm(kb + 9 * i)) * xs[j];
-    }
-#pragma unroll
     for (int i = 0; i < 4; ++i) stv(d.f0s + 12 * (size_t)e, i, f0acc[i]);
-    // plasticity: total strain B (R^T p - x0), elastic = total - plastic
-    float rx[12];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const f3 dd = RT * ps[i] - xs[i];
-        rx[3 * i] = dd.x, rx[3 * i + 1] = dd.y, rx[3 * i + 2] = dd.z;
-    }
-    // B (6 x 12, entry (i, k) at i + 6 k) in memory order, 16 bytes per load
-    const float4* B4 = reinterpret_cast<const float4*>(d.B + 72 * (size_t)e);
+    // plasticity: total strain B (R^T p - x0), elastic = total - plastic;
+    // each strain sums over the vertices' coordinates in order
     float* ep = d.eps + 6 * (size_t)e;
     float plastic[6], elastic[6], bacc[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int k2 = 0; k2 < 6; ++k2) {  // two columns k = 2 k2, 2 k2 + 1: 12 floats
-        float bb[12];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            const float4 t4 = B4[3 * k2 + q];
-            bb[4 * q] = t4.x, bb[4 * q + 1] = t4.y, bb[4 * q + 2] = t4.z, bb[4 * q + 3] = t4.w;
-        }
-#pragma unroll
-        for (int h2 = 0; h2 < 2; ++h2)
-#pragma unroll
-            for (int i = 0; i < 6; ++i) bacc[i] += bb[6 * h2 + i] * rx[2 * k2 + h2];
+    for (int i = 0; i < 4; ++i) {
+        const f3 r = RT * ps[i] - xs[i], g = sh.g[i];
+        bacc[0] += g.x * r.x;
+        bacc[1] += g.y * r.y;
+        bacc[2] += g.z * r.z;
+        bacc[3] += g.y * r.x;
+        bacc[3] += g.x * r.y;
+        bacc[4] += g.z * r.x;
+        bacc[4] += g.x * r.z;
+        bacc[5] += g.z * r.y;
+        bacc[5] += g.y * r.z;
     }
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
@@ -245,46 +317,57 @@ __global__ void k_sb_elements(SoftDev d, float h, float inv_h)
     }
 #pragma unroll
     for (int i = 0; i < 6; ++i) ep[i] = plastic[i];
-    // P (12 x 6, entry (3 i + r, k) at 3 i + r + 12 k) in memory order
-    const float4* P4 = reinterpret_cast<const float4*>(d.P + 72 * (size_t)e);
-    float pc[12] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    // P = V B^T D: one product an entry, summed over the strains in order
+    const float L = d.lambda, M = d.mu, T = d.lambda2mu, V = sh.vol;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        float pp[12];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            const float4 t4 = P4[3 * k + q];
-            pp[4 * q] = t4.x, pp[4 * q + 1] = t4.y, pp[4 * q + 2] = t4.z, pp[4 * q + 3] = t4.w;
-        }
-#pragma unroll
-        for (int m = 0; m < 12; ++m) pc[m] += pp[m] * plastic[k];
+    for (int i = 0; i < 4; ++i) {
+        const f3 g = sh.g[i];
+        f3 pc;
+        pc.x = ((((0.0f + ((g.x * T) * V) * plastic[0]) + ((g.x * L) * V) * plastic[1]) +
+                 ((g.x * L) * V) * plastic[2]) + ((g.y * M) * V) * plastic[3]) + ((g.z * M) * V) * plastic[4];
+        pc.y = ((((0.0f + ((g.y * L) * V) * plastic[0]) + ((g.y * T) * V) * plastic[1]) +
+                 ((g.y * L) * V) * plastic[2]) + ((g.x * M) * V) * plastic[3]) + ((g.z * M) * V) * plastic[5];
+        pc.z = ((((0.0f + ((g.z * L) * V) * plastic[0]) + ((g.z * L) * V) * plastic[1]) +
+                 ((g.z * T) * V) * plastic[2]) + ((g.x * M) * V) * plastic[4]) + ((g.y * M) * V) * plastic[5];
+        stv(d.fps + 12 * (size_t)e, i, R * pc);
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) stv(d.fps + 12 * (size_t)e, i, R * mk(pc[3 * i], pc[3 * i + 1], pc[3 * i + 2]));
 }
 
-// One warp per node.  The node's incidences are taken 32 at a time: each
+// L lanes per node: 8 or 16 where the node has no more incidences and slots
+// than that, else a warp.  The node's incidences are taken L at a time: each
 // lane forms its element's four R Ke_ij R^T blocks (and f0, f_plastic terms)
-// into shared memory; then each lane owns up to four of the row's slots and
-// adds, in incidence (= element) order, every block that lands on them --
-// the reference's K(vi, vj) += R Ke R^T order, so the row is the same float
-// for float.  K p, b and A follow as in the reference (:359-377), the serial
-// sums on lane 0.
+// into shared memory, and notes in a mask per (block of the element, slot of
+// the row) which slots they land on; then each lane owns one of the row's
+// slots and adds its blocks in incidence (= element) order, taking the set
+// bits of its masks -- the reference's K(vi, vj) += R Ke R^T order, so the row
+// is the same float for float.  K p, b and A follow as in the reference
+// (:359-377), the serial sums with a lane per component.
+//
+// Bound: instruction issue.  A 40^3 block's nodes have 8 or 24 incidences and
+// 7 or 19 slots, a slot about 6 of a chunk's blocks; before the masks every
+// lane compared all of them with its slot and the adds of different slots ran
+// one after another.  A 40^3 block: 320 us; with the masks 225; with the
+// element matrices formed here 209; with 8 and 16
+// lanes a narrow node 170 (its launches together).
 constexpr int kAsmWarps = 4;
 constexpr uint32_t kMaxRowSlots = 128;  // slot ids are 7 bits wide
+constexpr int kAsmStride = 37;          // words between two lanes' blocks: odd, so that a warp's banks differ
 
-__global__ void __launch_bounds__(32 * kAsmWarps, 8) k_sb_assemble(SoftDev d, float h)
+template <int L>
+__global__ void __launch_bounds__(32 * kAsmWarps, 6) k_sb_assemble(SoftDev d, const uint32_t* nodes, uint32_t count, float h)
 {
-    __shared__ __align__(16) float sX[kAsmWarps][32 * 4 * 9];   // element blocks of one chunk
-    __shared__ uint8_t sSlot[kAsmWarps][32 * 4];
-    __shared__ float sF[kAsmWarps][32 * 6];       // f0 and f_plastic terms of one chunk
-    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    const uint32_t i = blockIdx.x * kAsmWarps + w;
-    if (i >= d.n) return;  // whole warps leave together
-    float* X = sX[w];
-    uint8_t* SL = sSlot[w];
-    float* F = sF[w];
-    const uint32_t r0 = d.rowptr[i], deg = d.rowptr[i + 1] - r0;
+    __shared__ float sX[kAsmWarps][32 * kAsmStride];  // element blocks of one chunk
+    __shared__ uint32_t sM[kAsmWarps][4][32];         // per block of the element and slot: the lanes that land there
+    __shared__ float sF[kAsmWarps][6][33];            // f0 and f_plastic terms of one chunk, then K p
+    const uint32_t lane = threadIdx.x & (L - 1), w = threadIdx.x >> 5;  // lane of the node's L
+    const uint32_t at = threadIdx.x & 31u, first = at - lane;           // of the warp; the node's first
+    const uint32_t item = (blockIdx.x * 32u * kAsmWarps + threadIdx.x) / L;
+    if ((item & ~(32u / L - 1u)) >= count) return;  // whole warps leave together
+    const bool real = item < count;
+    const uint32_t i = nodes[real ? item : count - 1u];
+    float* X = sX[w] + kAsmStride * first;
+    float(*F)[33] = sF[w];
+    const uint32_t r0 = d.rowptr[i], deg = real ? d.rowptr[i + 1] - r0 : 0u;
     const float m = d.mass[i];
     const m3 M = diag3(m);
     // A = (M + h C) + (h h) K on the diagonal, 0 + (h h) K elsewhere
@@ -292,75 +375,77 @@ __global__ void __launch_bounds__(32 * kAsmWarps, 8) k_sb_assemble(SoftDev d, fl
     const float cd = d.damping[i] * m;
     const uint32_t dg = d.diag[i] - r0;
     float* vals = d.vals + 9 * (size_t)r0;
-    f3 f0 = zero3(), fp = zero3(), kp = zero3();
-    const uint32_t q0 = d.inc_ptr[i], q1 = d.inc_ptr[i + 1];
-    // Each lane owns one slot of a group of 32; a row wider than 32 slots
-    // (rare) takes the incidences again for each further group, so one
-    // accumulator suffices and the kernel keeps to 64 registers.  Groups run
-    // from the last down, so lane 0 can add K p in the row list's order
-    // (newest first touch first: slot deg-1 down to 0) as they finish.
-    for (uint32_t g = (deg + 31u) / 32u; g-- > 0;) {
+    float force = 0.0f;           // lanes 0-2: f0, lanes 3-5: f_plastic
+    float kp = 0.0f;              // lanes 0-2: K p
+    const uint32_t q0 = d.inc_ptr[i], q1 = real ? d.inc_ptr[i + 1] : q0;
+    // Each lane owns one slot of a group of L; with L = 32 a row wider than
+    // that (rare) takes the incidences again for each further group (fewer
+    // lanes: the node has at most L incidences and L slots).  Groups run from
+    // the last down, so K p can be added in the row list's order (newest
+    // first touch first: slot deg-1 down to 0) as they finish.
+    for (uint32_t g = L == 32 ? (deg + 31u) / 32u : 1u; g-- > 0;) {
         const uint32_t slot = lane + 32u * g;
         m3 acc = mzero();
-        for (uint32_t qb = q0; qb < q1; qb += 32u) {
-            const uint32_t cnt = min(32u, q1 - qb);
+        uint32_t qb = q0;
+        do {
+            const uint32_t cnt = min((uint32_t)L, q1 - qb);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sM[w][j][at] = 0u;
+            __syncwarp();
             if (lane < cnt) {
                 const uint32_t e = d.inc_elem[qb + lane], meta = d.inc_meta[qb + lane];
                 const uint32_t li = meta & 3u;
-                const m3 R = ldm(d.R + 9 * (size_t)e);
+                const m3 R = load_rotation(d.R + 3 * (size_t)e);
                 const m3 RT = transpose(R);
-                // Ke is symmetric and stored so: a block below the diagonal
-                // is the exact transpose of the one above it.  So the node's
-                // blocks Ke(li, j) are the transposes of Ke(j, li), j != li,
-                // which lie together, 144 bytes from 36 li on: nine 16-byte
-                // loads instead of four scattered 36-byte blocks.
-                // They are staged in the lane's own 36 floats of X and
-                // replaced there by the products, block by block.
-                const float4* K4 = reinterpret_cast<const float4*>(d.Ke + 144 * (size_t)e + 36 * li);
-                float4* X4 = reinterpret_cast<float4*>(X + 36 * lane);
-#pragma unroll 3
-                for (int q = 0; q < 9; ++q) X4[q] = K4[q];
+                Shape sh;
+                load_shape(d.shape + 3 * (size_t)e, sh);
+                const f3 gl = li == 0 ? sh.g[0] : li == 1 ? sh.g[1] : li == 2 ? sh.g[2] : sh.g[3];
 #pragma unroll
                 for (uint32_t j = 0; j < 4; ++j) {
-                    SL[4 * lane + j] = (uint8_t)((meta >> (4 + 7 * j)) & 127u);
-                    float* xb = X + 36 * lane + 9 * j;
-                    // Ke(li, j): Ke(j, li) itself on the diagonal, else its transpose
-                    if (j == li) stm(xb, mmul(mmul(R, ldm(xb)), RT));
-                    else stm(xb, mmul(mmul(R, transpose(ldm(xb))), RT));
+                    // Ke(li, j): below the diagonal the transpose of Ke(j, li)
+                    const bool lower = li > j;
+                    const m3 U = stiffness_block(d, lower ? sh.g[j] : gl, lower ? gl : sh.g[j], sh.vol);
+                    const m3 K{f3{U.x.x, lower ? U.y.x : U.x.y, lower ? U.z.x : U.x.z},
+                               f3{lower ? U.x.y : U.y.x, U.y.y, lower ? U.z.y : U.y.z},
+                               f3{lower ? U.x.z : U.z.x, lower ? U.y.z : U.z.y, U.z.z}};
+                    stm(X + kAsmStride * lane + 9 * j, mmul(mmul(R, K), RT));
+                    const uint32_t t = ((meta >> (4 + 7 * j)) & 127u) - 32u * g;
+                    if (t < (uint32_t)L) atomicOr(&sM[w][j][first + t], 1u << lane);
                 }
                 if (g == 0) {
                     const f3 a = ldv(d.f0s + 12 * (size_t)e, li), b = ldv(d.fps + 12 * (size_t)e, li);
-                    F[6 * lane] = a.x; F[6 * lane + 1] = a.y; F[6 * lane + 2] = a.z;
-                    F[6 * lane + 3] = b.x; F[6 * lane + 4] = b.y; F[6 * lane + 5] = b.z;
+                    F[0][at] = a.x, F[1][at] = a.y, F[2][at] = a.z;
+                    F[3][at] = b.x, F[4][at] = b.y, F[5][at] = b.z;
                 }
             }
             __syncwarp();
             // every block that lands on this slot, in incidence (= element) order
-            if (slot < deg)
-                for (uint32_t q = 0; q < cnt; ++q)
-#pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j)
-                        if (SL[4 * q + j] == slot) acc = acc + ldm(X + 9 * (4 * q + j));
-            if (g == 0 && lane == 0)
-                for (uint32_t q = 0; q < cnt; ++q) {
-                    f0 = f0 + mk(F[6 * q], F[6 * q + 1], F[6 * q + 2]);
-                    fp = fp + mk(F[6 * q + 3], F[6 * q + 4], F[6 * q + 5]);
-                }
+            // (an element's four nodes are four slots: one block a lane at most)
+            const uint32_t m0 = sM[w][0][at], m1 = sM[w][1][at], m2 = sM[w][2][at], m3_ = sM[w][3][at];
+            for (uint32_t left = m0 | m1 | m2 | m3_; left; left &= left - 1u) {
+                const uint32_t q = (uint32_t)__ffs(left) - 1u, bit = left & (0u - left);
+                const uint32_t j = (m1 & bit) ? 1u : (m2 & bit) ? 2u : (m3_ & bit) ? 3u : 0u;
+                acc = acc + ldm(X + kAsmStride * q + 9 * j);
+            }
+            if (g == 0 && lane < 6)
+                for (uint32_t q = 0; q < cnt; ++q) force = force + F[lane][first + q];
             __syncwarp();
-        }
+            qb += (uint32_t)L;
+        } while (L == 32 && qb < q1);
         f3 kx = zero3();
         if (slot < deg) kx = acc * ldv(d.x, d.cols[r0 + slot]);  // this slot's K_k x_col
-        for (uint32_t l = min(31u, deg - 1u - 32u * g) + 1u; l-- > 0;) {
-            const f3 t = mk(__shfl_sync(0xffffffffu, kx.x, l), __shfl_sync(0xffffffffu, kx.y, l),
-                            __shfl_sync(0xffffffffu, kx.z, l));
-            if (lane == 0) kp = kp + t;
-        }
+        F[0][at] = kx.x, F[1][at] = kx.y, F[2][at] = kx.z;
+        __syncwarp();
+        if (lane < 3)
+            for (uint32_t l = min(32u, deg - 32u * g); l-- > 0;) kp = kp + F[lane][first + l];
+        __syncwarp();
         if (slot < deg) {
             m3 a;
             if (slot == dg) a = (M + h * diag3(cd)) + hh * acc;
             else a = mzero() + hh * acc;
-            stm(vals + 9 * slot, a);
-            if (d.sell_vals) {
+            if (!d.sell_vals) {
+                stm(vals + 9 * slot, a);
+            } else {
                 // the SELL copy keeps the diagonal block in slot 0, then the rest in order
                 const uint32_t ri = d.sell_inv[i];
                 const uint32_t ss = slot == dg ? 0u : slot < dg ? slot + 1u : slot;
@@ -376,22 +461,43 @@ __global__ void __launch_bounds__(32 * kAsmWarps, 8) k_sb_assemble(SoftDev d, fl
             }
         }
     }
-    if (lane == 0) {
+    auto from = [&](float v, int k) { return __shfl_sync(0xffffffffu, v, k, L); };
+    const f3 f0 = mk(from(force, 0), from(force, 1), from(force, 2));
+    const f3 fp = mk(from(force, 3), from(force, 4), from(force, 5));
+    const f3 kpv = mk(from(kp, 0), from(kp, 1), from(kp, 2));
+    if (lane == 0 && real) {
         const bool dyn = d.type[i] == 2;
         const f3 f0n = mk(-f0.x, -f0.y, -f0.z);
         f3 fe = ldv(d.f, i);
         if (dyn) fe = fe + m * mk(d.gx, d.gy, d.gz);
         const f3 mv = zero3() + M * ldv(d.v, i);
-        const f3 bi = mv - h * ((kp + f0n) - (fp + fe));
-        stv(d.b, i, bi);
-        d.S[i] = dyn ? 1.0f : 0.0f;
-        if (d.sell_vals) {
+        const f3 bi = mv - h * ((kpv + f0n) - (fp + fe));
+        if (!d.sell_vals) {
+            stv(d.b, i, bi);
+            d.S[i] = dyn ? 1.0f : 0.0f;
+        } else {
             const uint32_t ri = d.sell_inv[i];
             st3(d.sb_b, d.n, ri, bi);
             st3(d.sb_x0, d.n, ri, ldv(d.v, i));
             d.sb_type[ri] = d.type[i];
         }
     }
+}
+
+// The assembly of every node, in its three classes.
+cudaError_t launch_sb_assemble(const SoftDev& d, float h, cudaStream_t s)
+{
+    const uint32_t* p = d.asm_nodes;
+    const uint32_t per = 32 * kAsmWarps;
+    auto blocks = [&](uint32_t count, uint32_t lanes) { return (count * lanes + per - 1) / per; };
+    uint32_t launches = 0;
+    if (d.asm_count[0]) k_sb_assemble<32><<<blocks(d.asm_count[0], 32), per, 0, s>>>(d, p, d.asm_count[0], h), ++launches;
+    p += d.asm_count[0];
+    if (d.asm_count[1]) k_sb_assemble<16><<<blocks(d.asm_count[1], 16), per, 0, s>>>(d, p, d.asm_count[1], h), ++launches;
+    p += d.asm_count[1];
+    if (d.asm_count[2]) k_sb_assemble<8><<<blocks(d.asm_count[2], 8), per, 0, s>>>(d, p, d.asm_count[2], h), ++launches;
+    count_launches(launches);
+    return cudaGetLastError();
 }
 
 // b3BroadPhase::MoveProxy for node i's proxy (b3SoftBodyNode::Synchronize,
@@ -935,10 +1041,10 @@ b3g_status b3g_softbody_create(uint32_t vertex_count, const float* vertices, uin
     const uint32_t grid = csr_grid(n);
     size_t bytes = 0;
     const size_t sizes[] = {vec,       vec,       vec,       vec,          (size_t)n * 4, (size_t)n * 4, (size_t)n,
-                            (size_t)t * 16, (size_t)t * 576, (size_t)t * 36, (size_t)t * 288, (size_t)t * 288,
-                            (size_t)t * 16, (size_t)t * 24, (size_t)t * 36, (size_t)t * 48, (size_t)t * 48,
+                            (size_t)t * 16, (size_t)t * 48,
+                            (size_t)t * 16, (size_t)t * 24, (size_t)t * 48, (size_t)t * 48, (size_t)t * 48,
                             (size_t)(n + 1) * 4, (size_t)nnz * 4, (size_t)n * 4, (size_t)nnz * 36,
-                            (size_t)(n + 1) * 4, (size_t)t * 16, (size_t)t * 16, vec, (size_t)n * 4, vec,
+                            (size_t)(n + 1) * 4, (size_t)t * 16, (size_t)t * 16, (size_t)n * 4, vec, (size_t)n * 4, vec,
                             csr_scratch_bytes(n, grid)};
     for (size_t s : sizes) bytes += al(s);
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
@@ -971,17 +1077,14 @@ b3g_status b3g_softbody_create(uint32_t vertex_count, const float* vertices, uin
     d.type = (uint8_t*)take(n);
     uint4* tv = (uint4*)take((size_t)t * 16);
     d.tets = tv;
-    float* Ke = (float*)take((size_t)t * 576);
-    d.Ke = Ke;
-    float* invE = (float*)take((size_t)t * 36);
-    d.invE = invE;
-    float* Bm = (float*)take((size_t)t * 288);
-    d.B = Bm;
-    float* Pm = (float*)take((size_t)t * 288);
-    d.P = Pm;
+    float4* shape = (float4*)take((size_t)t * 48);
+    d.shape = shape;
+    d.lambda = P.lambda;
+    d.mu = P.mu;
+    d.lambda2mu = P.lambda2mu;
     d.q = (float4*)take((size_t)t * 16);
     d.eps = (float*)take((size_t)t * 24);
-    d.R = (float*)take((size_t)t * 36);
+    d.R = (float4*)take((size_t)t * 48);
     d.f0s = (float*)take((size_t)t * 48);
     d.fps = (float*)take((size_t)t * 48);
     uint32_t* rowptr = (uint32_t*)take((size_t)(n + 1) * 4);
@@ -997,6 +1100,20 @@ b3g_status b3g_softbody_create(uint32_t vertex_count, const float* vertices, uin
     d.inc_elem = inc_elem;
     uint32_t* inc_meta = (uint32_t*)take((size_t)t * 16);
     d.inc_meta = inc_meta;
+    uint32_t* asm_nodes = (uint32_t*)take((size_t)n * 4);
+    d.asm_nodes = asm_nodes;
+    // three launches by the lanes a node needs; a body of few nodes leaves the
+    // GPU idle anyway and takes one (512 nodes: 138 us a step against 143,
+    // 9,261: 206 against 202)
+    std::vector<uint32_t> by_lanes;
+    by_lanes.reserve(n);
+    for (int cls = 0; cls < 3; ++cls) {
+        d.asm_count[cls] = 0;
+        for (uint32_t i = 0; i < n; ++i) {
+            const uint32_t most = std::max(P.inc_ptr[i + 1] - P.inc_ptr[i], P.rowptr[i + 1] - P.rowptr[i]);
+            if ((n < 8192 || most > 16 ? 0 : most > 8 ? 1 : 2) == cls) by_lanes.push_back(i), d.asm_count[cls] += 1;
+        }
+    }
     d.b = (float*)take(vec);
     d.S = (float*)take((size_t)n * 4);
     d.xsol = (float*)take(vec);
@@ -1015,11 +1132,11 @@ b3g_status b3g_softbody_create(uint32_t vertex_count, const float* vertices, uin
         const void* src;
         size_t bytes;
     } ups[] = {{rest, vertices, vec}, {d.x, vertices, vec}, {mass, P.mass.data(), (size_t)n * 4},
-               {tv, tets4.data(), (size_t)t * 16}, {Ke, P.Ke.data(), (size_t)t * 576},
-               {invE, P.invE.data(), (size_t)t * 36}, {Bm, P.B.data(), (size_t)t * 288},
-               {Pm, P.P.data(), (size_t)t * 288}, {d.q, q0.data(), (size_t)t * 16},
+               {tv, tets4.data(), (size_t)t * 16}, {shape, P.shape.data(), (size_t)t * 48},
+               {d.q, q0.data(), (size_t)t * 16},
                {rowptr, P.rowptr.data(), (size_t)(n + 1) * 4}, {cols, P.cols.data(), (size_t)nnz * 4},
                {dg, P.diag.data(), (size_t)n * 4}, {inc_ptr, P.inc_ptr.data(), (size_t)(n + 1) * 4},
+               {asm_nodes, by_lanes.data(), (size_t)n * 4},
                {inc_elem, P.inc_elem.data(), (size_t)t * 16}, {inc_meta, P.inc_meta.data(), (size_t)t * 16},
                {d.type, types.data(), (size_t)n}};
     for (const Up& u : ups)
@@ -1183,10 +1300,11 @@ b3g_status b3g_softbody_step(b3g_softbody* b, float dt, uint32_t velocity_iterat
             const b3g_status es = ensure_sell(b);
             if (es != B3G_OK) return es;
         }
-        k_sb_elements<<<blocks_for(d.t), kBlock, 0, s>>>(d, dt, 1.0f / dt);
-        k_sb_assemble<<<(d.n + kAsmWarps - 1) / kAsmWarps, 32 * kAsmWarps, 0, s>>>(d, dt);
-        count_launches(2);
-        SB_TRY(cudaGetLastError());
+        k_sb_elements<<<(d.t + 127) / 128, 128, 0, s>>>(d, dt, 1.0f / dt);
+        SoftDev w = d;  // the system goes where this step's CG reads it
+        if (!b->persistent) w.sell_vals = nullptr;
+        SB_TRY(launch_sb_assemble(w, dt, s));
+        count_launches(1);
         const b3g_status r = b->persistent ? persistent_cg(b, s, &h) : csr_run(b->cs, &b->opts, s, &h);
         if (r != B3G_OK) return r;
         if (d.nhull) {
@@ -1411,10 +1529,11 @@ b3g_status b3g_softbody_export_system(b3g_softbody* b, float dt, uint32_t capaci
     std::vector<float> q(4 * (size_t)d.t), eps(6 * (size_t)d.t);
     b3g_status r = b3g_softbody_read_elements(b, q.data(), eps.data());
     if (r != B3G_OK) return r;
-    k_sb_elements<<<blocks_for(d.t), kBlock, 0, s>>>(d, dt, 1.0f / dt);
-    k_sb_assemble<<<(d.n + kAsmWarps - 1) / kAsmWarps, 32 * kAsmWarps, 0, s>>>(d, dt);
-    count_launches(2);
-    SB_TRY(cudaGetLastError());
+    SoftDev w = d;
+    w.sell_vals = nullptr;  // the row lists
+    k_sb_elements<<<(d.t + 127) / 128, 128, 0, s>>>(d, dt, 1.0f / dt);
+    SB_TRY(launch_sb_assemble(w, dt, s));
+    count_launches(1);
     std::vector<float> v(9 * (size_t)d.nnz);
     SB_TRY(cudaMemcpyAsync(v.data(), d.vals, v.size() * 4, cudaMemcpyDeviceToHost, s));
     SB_TRY(cudaMemcpyAsync(rhs, d.b, 3 * (size_t)d.n * 4, cudaMemcpyDeviceToHost, s));

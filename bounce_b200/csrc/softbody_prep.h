@@ -12,11 +12,11 @@ namespace b3g {
 struct SoftBodyPrep {
     uint32_t n = 0, t = 0;
     std::vector<float> mass;        // n
-    // per element, in b3SoftBodyElement's arithmetic
-    std::vector<float> Ke;          // 144: 16 blocks (block i + 4 j), 9 floats column-major
-    std::vector<float> invE;        // 9
-    std::vector<float> B;           // 72 (6 x 12, column-major)
-    std::vector<float> P;           // 72 (12 x 6, column-major)
+    // per element, in b3SoftBodyElement's arithmetic: the inverse of its edge
+    // matrix (9 floats, column-major), its volume and two zeros.  The element
+    // matrices Ke, B and P follow from these and the material (softbody.cu).
+    std::vector<float> shape;       // 12
+    float lambda = 0.0f, mu = 0.0f, lambda2mu = 0.0f;  // of the isotropic elasticity matrix
     // block rows: row i's columns in the order the element loop first
     // touches them (the reverse of the stiffness matrix's row list)
     std::vector<uint32_t> rowptr;   // n + 1

@@ -344,3 +344,22 @@ def test_softbody_coplanar_hulls_contact_order(b3g, port):
         nodes = np.nonzero(oact)[0] % n
         multi = max(multi, int((np.bincount(nodes, minlength=n) >= 2).sum()) if nodes.size else 0)
     assert multi > 0
+
+
+@pytest.mark.parametrize("size", [(1, 1, 1), (2, 3, 1), (24, 18, 19)])
+def test_softbody_assembly_lane_classes(b3g, port, size):
+    """A and b of an irregularly deformed block are the oracle's floats, below
+    and above the size from which narrow nodes share a warp."""
+    scene = b3g.pinned_block_scene(*size, 0.1)
+    gpu, ora = _pair(b3g, port, scene)
+    rng = np.random.default_rng(4)
+    x = (scene.vertices + rng.normal(0.0, 0.004, scene.vertices.shape)).astype(np.float32)
+    v = rng.normal(0.0, 0.3, x.shape).astype(np.float32)
+    v[scene.static_nodes] = 0.0
+    gpu.write_state(x, v)
+    ora.set_state(x=x, v=v)
+    a, b = gpu.system(scene.dt), ora.system(scene.dt)
+    for key in ("rowptr", "cols"):
+        assert np.array_equal(a[key], b[key])
+    for key in ("vals", "b"):
+        assert np.array_equal(a[key], b[key]), key
