@@ -41,6 +41,10 @@ constexpr float kMaxCorrection = 0.2f;    // B3_MAX_LINEAR_CORRECTION
 constexpr float kBaum = 0.1f;             // B3_BAUMGARTE
 constexpr float kEpsilon = 1.1920929e-7f; // B3_EPSILON (FLT_EPSILON)
 constexpr int kSolveThreads = 1024;
+constexpr int kSharedThreads = 512;       // 128 registers: the walking warp must not spill
+constexpr int kMaxStretches = 256;        // stretches of levels a contact solve brings in
+constexpr uint32_t kSolveSmem = 220 * 1024;
+constexpr uint32_t kSharedParticles = 8192;  // at most 96 KB of the solve's shared memory a plane
 constexpr uint32_t kMaxBodyContacts = kMaxSpheres;
 
 __device__ __forceinline__ f3 neg(f3 v) { return mk(-v.x, -v.y, -v.z); }
@@ -241,11 +245,11 @@ __device__ int body_order(const ClothDev& c, uint32_t i, int* order)
 }
 
 // WarmStartBodyContactConstraints (cloth_contact_solver.cpp:264-307)
-__device__ void body_warm_start(const ClothDev& c, uint32_t i, const int* order, int k)
+__device__ void body_warm_start(const ClothDev& c, float* v, uint32_t i, const int* order, int k)
 {
     const uint32_t n = c.n, nn = c.nsph * n;
     const float mA = 1.0f / c.mass[i];
-    f3 vel = ld3(c.v, n, i);
+    f3 vel = ld3(v, n, i);
     for (int a = 0; a < k; ++a) {
         const uint32_t q = order[a] * n + i;
         const f3 nrm = ld3(c.c_normal, nn, q), t1 = ld3(c.c_t1, nn, q), t2 = ld3(c.c_t2, nn, q);
@@ -254,15 +258,15 @@ __device__ void body_warm_start(const ClothDev& c, uint32_t i, const int* order,
         const f3 P1 = c.c_imp[nn + q] * t1, P2 = c.c_imp[2 * nn + q] * t2;
         vel = vel - mA * (P1 + P2);
     }
-    st3(c.v, n, i, vel);
+    st3(v, n, i, vel);
 }
 
 // SolveBodyContactVelocityConstraints (cloth_contact_solver.cpp:388-472)
-__device__ void body_velocity(const ClothDev& c, uint32_t i, const int* order, int k)
+__device__ void body_velocity(const ClothDev& c, float* v, uint32_t i, const int* order, int k)
 {
     const uint32_t n = c.n, nn = c.nsph * n;
     const float mA = 1.0f / c.mass[i];
-    f3 vel = ld3(c.v, n, i);
+    f3 vel = ld3(v, n, i);
     for (int a = 0; a < k; ++a) {
         const int sidx = order[a];
         const uint32_t q = sidx * n + i;
@@ -313,16 +317,16 @@ __device__ void body_velocity(const ClothDev& c, uint32_t i, const int* order, i
         c.c_imp[nn + q] = tix;
         c.c_imp[2 * nn + q] = tiy;
     }
-    st3(c.v, n, i, vel);
+    st3(v, n, i, vel);
 }
 
 // SolveBodyContactPositionConstraints (cloth_contact_solver.cpp:620-718);
 // returns the smallest separation
-__device__ float body_position(const ClothDev& c, uint32_t i, const int* order, int k)
+__device__ float body_position(const ClothDev& c, float* x, uint32_t i, const int* order, int k)
 {
     const uint32_t n = c.n, nn = c.nsph * n;
     const float mA = 1.0f / c.mass[i];
-    f3 pos = ld3(c.x, n, i);
+    f3 pos = ld3(x, n, i);
     float min_sep = 0.0f;
     for (int a = 0; a < k; ++a) {
         const int sidx = order[a];
@@ -339,7 +343,7 @@ __device__ float body_position(const ClothDev& c, uint32_t i, const int* order, 
         const f3 P = impulse * nA;
         pos = pos - mA * P;
     }
-    st3(c.x, n, i, pos);
+    st3(x, n, i, pos);
     return min_sep;
 }
 
@@ -403,19 +407,19 @@ __device__ __forceinline__ void apply(const TriCon& x, float lambda, f3 u, Quad&
 }
 
 // WarmStartTriangleContactConstraints (cloth_contact_solver.cpp:309-386)
-__device__ void tri_warm_start(const ClothDev& c, const TriCon& x)
+__device__ __forceinline__ void tri_warm_start(float* v, uint32_t n, const TriCon& x)
 {
-    Quad q = load_quad(c.v, c.n, x);
+    Quad q = load_quad(v, n, x);
     apply(x, x.ni, mk(x.nx, x.ny, x.nz), q);
     apply(x, x.ti1, mk(x.t1x, x.t1y, x.t1z), q);
     apply(x, x.ti2, mk(x.t2x, x.t2y, x.t2z), q);
-    store_quad(c.v, c.n, x, q);
+    store_quad(v, n, x, q);
 }
 
 // SolveTriangleContactVelocityConstraints (cloth_contact_solver.cpp:474-596)
-__device__ void tri_velocity(const ClothDev& c, TriCon& x)
+__device__ __forceinline__ void tri_velocity(float* v, uint32_t n, TriCon& x)
 {
-    Quad q = load_quad(c.v, c.n, x);
+    Quad q = load_quad(v, n, x);
     {
         const f3 nrm = mk(x.nx, x.ny, x.nz);
         const f3 vCB = (x.wB * q.b + x.wC * q.c) + x.wD * q.d;
@@ -427,6 +431,7 @@ __device__ void tri_velocity(const ClothDev& c, TriCon& x)
         impulse = x.ni - old;
         apply(x, impulse, nrm, q);
     }
+#pragma unroll
     for (int dir = 0; dir < 2; ++dir) {
         const float hi = x.friction * x.ni;
         const float lo = -hi;
@@ -442,13 +447,13 @@ __device__ void tri_velocity(const ClothDev& c, TriCon& x)
         impulse = acc - old;
         apply(x, impulse, u, q);
     }
-    store_quad(c.v, c.n, x, q);
+    store_quad(v, n, x, q);
 }
 
 // SolveTriangleContactPositionConstraints (cloth_contact_solver.cpp:720-794)
-__device__ float tri_position(const ClothDev& c, const TriCon& x)
+__device__ __forceinline__ float tri_position(float* p, uint32_t n, const TriCon& x)
 {
-    Quad q = load_quad(c.x, c.n, x);
+    Quad q = load_quad(p, n, x);
     const f3 cB = (x.wB * q.b + x.wC * q.c) + x.wD * q.d;
     f3 nrm = cB - q.a;
     const float distance = normalize(nrm);
@@ -459,7 +464,120 @@ __device__ float tri_position(const ClothDev& c, const TriCon& x)
     const float K = ((x.mA + x.mB * x.wB * x.wB) + x.mC * x.wC * x.wC) + x.mD * x.wD * x.wD;
     const float impulse = K > 0.0f ? -C / K : 0.0f;
     apply(x, impulse, nrm, q);
-    store_quad(c.x, c.n, x, q);
+    store_quad(p, n, x, q);
+    return separation;
+}
+
+// The same three solves with a lane per component: lanes 3 g, 3 g + 1, 3 g + 2
+// of the warp hold x, y and z of contact g, so that a contact is a third of
+// the instructions long.  Every vector expression is the component's own, and
+// a dot product's three terms go to all three lanes and are added in order.
+constexpr uint32_t kLaneCons = 10;  // contacts of a warp
+struct LaneCon {
+    uint4 id;
+    float4 m, w;           // inverse masses; wB, wC, wD, friction
+    float4 imp;            // ni, ti1, ti2
+    float n, t1, t2, normal_mass, radius_a, radius_t;
+};
+__device__ __forceinline__ LaneCon lane_con(const TriCon* con, uint32_t comp)
+{
+    const float4* q = reinterpret_cast<const float4*>(con);
+    const float* f = reinterpret_cast<const float*>(con);
+    LaneCon x;
+    x.id = *reinterpret_cast<const uint4*>(q);
+    x.m = q[1];
+    x.w = q[2];
+    x.imp = q[6];
+    x.n = f[12 + comp];
+    x.normal_mass = f[15];
+    x.t1 = f[16 + comp];
+    x.radius_a = f[19];
+    x.t2 = f[20 + comp];
+    x.radius_t = f[23];
+    return x;
+}
+struct LaneQuad {
+    float a, b, c, d;
+};
+// One component of the plane at the contact's particles, and back.
+__device__ __forceinline__ LaneQuad lane_load(const float* p, const LaneCon& x)
+{
+    return LaneQuad{p[x.id.x], p[x.id.y], p[x.id.z], p[x.id.w]};
+}
+__device__ __forceinline__ void lane_store(float* p, const LaneCon& x, const LaneQuad& q)
+{
+    p[x.id.x] = q.a;
+    p[x.id.y] = q.b;
+    p[x.id.z] = q.c;
+    p[x.id.w] = q.d;
+}
+__device__ __forceinline__ void lane_apply(const LaneCon& x, float lambda, float u, LaneQuad& q)
+{
+    const float JA = -u, JB = x.w.x * u, JC = x.w.y * u, JD = x.w.z * u;
+    const float PA = lambda * JA, PB = lambda * JB, PC = lambda * JC, PD = lambda * JD;
+    q.a = q.a + x.m.x * PA;
+    q.b = q.b + x.m.y * PB;
+    q.c = q.c + x.m.z * PC;
+    q.d = q.d + x.m.w * PD;
+}
+// x + y + z of the contact's lanes, from the first of them on.
+__device__ __forceinline__ float lane_dot(float v, uint32_t first)
+{
+    const float x = __shfl_sync(0xffffffffu, v, first), y = __shfl_sync(0xffffffffu, v, first + 1u),
+                z = __shfl_sync(0xffffffffu, v, first + 2u);
+    return x + y + z;
+}
+__device__ __forceinline__ void lane_warm_start(LaneQuad& q, const LaneCon& x)
+{
+    lane_apply(x, x.imp.x, x.n, q);
+    lane_apply(x, x.imp.y, x.t1, q);
+    lane_apply(x, x.imp.z, x.t2, q);
+}
+__device__ __forceinline__ void lane_velocity(LaneQuad& q, LaneCon& x, uint32_t first)
+{
+    {
+        const float vCB = (x.w.x * q.b + x.w.y * q.c) + x.w.z * q.d;
+        const float Cdot = lane_dot((vCB - q.a) * x.n, first);
+        float impulse = -x.normal_mass * Cdot;
+        const float old = x.imp.x;
+        const float sum = x.imp.x + impulse;
+        x.imp.x = sum > 0.0f ? sum : 0.0f;
+        impulse = x.imp.x - old;
+        lane_apply(x, impulse, x.n, q);
+    }
+#pragma unroll
+    for (int dir = 0; dir < 2; ++dir) {
+        const float hi = x.w.w * x.imp.x;
+        const float lo = -hi;
+        const float u = dir == 0 ? x.t1 : x.t2;
+        float& acc = dir == 0 ? x.imp.y : x.imp.z;
+        const float vCB = (x.w.x * q.b + x.w.y * q.c) + x.w.z * q.d;
+        const float Cdot = lane_dot((vCB - q.a) * u, first);
+        float impulse = -x.normal_mass * Cdot;
+        const float old = acc;
+        const float a = acc + impulse;
+        const float m = a < hi ? a : hi;
+        acc = lo > m ? lo : m;
+        impulse = acc - old;
+        lane_apply(x, impulse, u, q);
+    }
+}
+__device__ __forceinline__ float lane_position(LaneQuad& q, const LaneCon& x, uint32_t first)
+{
+    const float cB = (x.w.x * q.b + x.w.y * q.c) + x.w.z * q.d;
+    float nrm = cB - q.a;
+    const float distance = sqrtf(lane_dot(nrm * nrm, first));  // normalize()
+    if (distance > kEpsilon) {
+        const float s = 1.0f / distance;
+        nrm = nrm * s;
+    }
+    const float separation = (distance - x.radius_a) - x.radius_t;
+    const float Cv = kBaum * (separation + kSlop);
+    const float m = Cv < 0.0f ? Cv : 0.0f;
+    const float C = -kMaxCorrection > m ? -kMaxCorrection : m;
+    const float K = ((x.m.x + x.m.y * x.w.x * x.w.x) + x.m.z * x.w.y * x.w.y) + x.m.w * x.w.z * x.w.z;
+    const float impulse = K > 0.0f ? -C / K : 0.0f;
+    lane_apply(x, impulse, nrm, q);
     return separation;
 }
 
@@ -476,16 +594,30 @@ __device__ __forceinline__ float dec_min(int i) { return __int_as_float(i >= 0 ?
 // out.  Triangle contacts run level by level: a contact's level is one more
 // than the highest level of an earlier active contact sharing a particle, so
 // each particle's updates come in list order.
-__global__ void __launch_bounds__(kSolveThreads) k_sc_solve(ClothDev c, SelfDev s, int cur)
+//
+// Bound: latency.  A fold chains thousands of contacts through shared
+// particles (two layers of 24^2: 3,082 contacts in 2,145 levels), and a level
+// is one contact's dependent arithmetic, about 60 operations a velocity sweep.
+// So SHARED (the particles' planes fit beside the buffers) keeps the plane
+// that a sweep works on in shared memory, stores the constraints in the order
+// of their levels, and while warp 0 walks one stretch of levels the other
+// warps bring the next into shared memory; warp 0 has a level's constraints in
+// registers before the level ahead of it is done, and runs a contact on three
+// lanes, one a component.  The fold above, a step: 19.5 ms with both in global
+// memory and a contact a lane, 9.8 in shared memory, 8.7 on three lanes (700
+// cycles a level of a velocity sweep, about 450 of them the chain itself).
+template <bool SHARED>
+__global__ void __launch_bounds__(SHARED ? kSharedThreads : kSolveThreads) k_sc_solve(ClothDev c, SelfDev s, int cur, uint32_t smem_bytes)
 {
-    extern __shared__ uint32_t last[];  // per particle: level of its latest contact
+    extern __shared__ __align__(16) uint32_t last[];  // per particle: level of its latest contact; then a plane
     __shared__ int s_min[2];
-    __shared__ uint32_t s_levels, s_width;
-    const uint32_t n = c.n, tid = threadIdx.x, nt = blockDim.x;
+    __shared__ uint32_t s_levels, s_width, s_chunks;
+    __shared__ uint32_t s_first[kMaxStretches + 1];   // first level of each stretch
+    const uint32_t n = c.n, tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u;
     StepScalars* sc = c.sc;
     const float h = sc->dt;
     const uint32_t A = s.counts[kCountActive];
-    const uint32_t* ls = s.level_start;
+    uint32_t* ls = s.level_start;
 
     for (uint32_t i = tid; i < n; i += nt) {
         const f3 dv = ld3(c.dv, n, i);
@@ -494,61 +626,168 @@ __global__ void __launch_bounds__(kSolveThreads) k_sc_solve(ClothDev c, SelfDev 
         st3(c.mx, n, i, dv);
         last[i] = 0;
     }
-    __syncthreads();
+    // the contacts' particles, in list order
     for (uint32_t a = tid; a < A; a += nt) {
-        const uint32_t k = s.active_idx[a];
-        tri_init(c, s.con[a], s.key[cur][k], s.w[cur][k], s.imp[cur][k]);
+        const uint2 key = s.key[cur][s.active_idx[a]];
+        const uint4 tv = c.tri[key.y];
+        TriCon& x = s.con[a];
+        x.ia = key.x, x.ib = tv.x, x.ic = tv.y, x.id = tv.z;
     }
+    for (uint32_t L = tid; L <= A + 1; L += nt) ls[L] = 0;
+    if (tid == 0) s_levels = s_width = 0u;
     __syncthreads();
-    if (tid == 0) {
-        // levels, then the contacts grouped by level (ascending within a level)
+    if (tid < 32u) {
+        // levels in list order: 32 contacts' particles a load
         uint32_t top = 0;
-        for (uint32_t a = 0; a < A; ++a) {
-            TriCon& x = s.con[a];
-            uint32_t L = last[x.ia];
-            L = last[x.ib] > L ? last[x.ib] : L;
-            L = last[x.ic] > L ? last[x.ic] : L;
-            L = last[x.id] > L ? last[x.id] : L;
-            L += 1;
-            last[x.ia] = last[x.ib] = last[x.ic] = last[x.id] = L;
-            x.pad = __uint_as_float(L);
-            top = L > top ? L : top;
+        for (uint32_t a0 = 0; a0 < A; a0 += 32u) {
+            uint4 id = make_uint4(0u, 0u, 0u, 0u);
+            if (a0 + lane < A) id = *reinterpret_cast<const uint4*>(&s.con[a0 + lane]);
+            uint32_t mine = 0;
+            for (uint32_t k = 0; k < 32u && a0 + k < A; ++k) {
+                const uint32_t ia = __shfl_sync(0xffffffffu, id.x, k), ib = __shfl_sync(0xffffffffu, id.y, k),
+                               ic = __shfl_sync(0xffffffffu, id.z, k), id4 = __shfl_sync(0xffffffffu, id.w, k);
+                const uint32_t L = max(max(last[ia], last[ib]), max(last[ic], last[id4])) + 1u;
+                __syncwarp();
+                if (lane < 4u) last[lane == 0 ? ia : lane == 1 ? ib : lane == 2 ? ic : id4] = L;
+                __syncwarp();
+                if (lane == k) mine = L;
+                top = max(top, L);
+            }
+            if (a0 + lane < A) {
+                s.con[a0 + lane].pad = __uint_as_float(mine);
+                atomicAdd(&ls[mine], 1u);
+            }
         }
-        uint32_t* lsw = s.level_start;
-        for (uint32_t L = 0; L <= top + 1; ++L) lsw[L] = 0;
-        for (uint32_t a = 0; a < A; ++a) lsw[__float_as_uint(s.con[a].pad)] += 1;
-        uint32_t width = 0;
-        for (uint32_t L = 1; L <= top; ++L) width = lsw[L] > width ? lsw[L] : width;
-        s_width = width;
-        for (uint32_t L = 1; L <= top; ++L) lsw[L] += lsw[L - 1];
-        lsw[top + 1] = A;
-        for (uint32_t a = A; a-- > 0;) s.by_level[--lsw[__float_as_uint(s.con[a].pad)]] = a;
-        s_levels = top;
-        s.counts[kCountLevels] = top;
+        if (lane == 0) s_levels = top;
     }
     __syncthreads();
     const uint32_t top = s_levels;
+    // the contacts grouped by level: inclusive sums, then every contact takes
+    // the last free place of its level (the order within a level is free)
+    uint32_t carry = 0;
+    for (uint32_t L0 = 0; L0 <= top; L0 += nt) {
+        const uint32_t v = L0 + tid <= top ? ls[L0 + tid] : 0u;
+        if (v) atomicMax(&s_width, v);
+        uint32_t sum;
+        const uint32_t before = block_scan(v, sum);
+        if (L0 + tid <= top) ls[L0 + tid] = carry + before + v;
+        carry += sum;
+    }
+    __syncthreads();
+    for (uint32_t a = tid; a < A; a += nt) s.by_level[atomicSub(&ls[__float_as_uint(s.con[a].pad)], 1u) - 1u] = a;
+    if (tid == 0) {
+        ls[top + 1] = A;
+        s.counts[kCountLevels] = top;
+    }
+    __syncthreads();
+    for (uint32_t j = tid; j < A; j += nt) {
+        const uint32_t k = s.active_idx[s.by_level[j]];
+        tri_init(c, s.con[j], s.key[cur][k], s.w[cur][k], s.imp[cur][k]);
+    }
     // Levels of at most 32 contacts run in warp 0 alone, with warp
     // barriers between levels; wider ones use the whole block.
     const bool narrow = s_width <= 32u;
-    const uint32_t lane = tid & 31u;
-    auto sweep = [&](auto&& fn) {
-        if (narrow) {
+    float* plane = reinterpret_cast<float*>(last);  // SHARED: the particles' v or x
+    const uint32_t plane_bytes = (12u * n + 15u) & ~15u;
+    const uint32_t room = SHARED ? (smem_bytes - plane_bytes) / (2u * (sizeof(TriCon) + 8u)) - 2u : 0u;  // a buffer
+    if (SHARED && narrow && tid == 0) {
+        // stretches of levels that fill a buffer; too many of them: from global memory
+        uint32_t L = 1, q = 0;
+        while (L <= top && q < (uint32_t)kMaxStretches) {
+            s_first[q++] = L;
+            uint32_t lo = L, hi = top;  // the last level whose contacts still fit
+            const uint32_t limit = ls[L] + room;
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi + 1u) / 2u;
+                if (ls[mid + 1] <= limit) lo = mid;
+                else hi = mid - 1u;
+            }
+            L = lo + 1u;
+        }
+        s_first[q] = L;
+        s_chunks = L > top ? q : 0u;
+    }
+    __syncthreads();
+    const uint32_t chunks = SHARED && narrow ? s_chunks : 0u;
+    TriCon* buf[2];
+    uint32_t* start[2];
+    buf[0] = reinterpret_cast<TriCon*>(reinterpret_cast<char*>(last) + plane_bytes);
+    buf[1] = buf[0] + (room + 2u);
+    start[0] = reinterpret_cast<uint32_t*>(buf[1] + (room + 2u));
+    start[1] = start[0] + (room + 2u);
+    // stretch q into its buffer, by threads first, first + step, ...
+    auto bring = [&](uint32_t q, uint32_t first, uint32_t step) {
+        const uint32_t L0 = s_first[q], L1 = s_first[q + 1], j0 = ls[L0], j1 = ls[L1];
+        const float4* from = reinterpret_cast<const float4*>(s.con + j0);
+        float4* to = reinterpret_cast<float4*>(buf[q & 1u]);
+        for (uint32_t k = first; k < (j1 - j0) * (uint32_t)(sizeof(TriCon) / 16); k += step) to[k] = __ldcg(from + k);
+        for (uint32_t k = first; k <= L1 - L0; k += step) start[q & 1u][k] = ls[L0 + k] - j0;
+    };
+    // Every contact once, in the levels' order, on the plane p: whole(p, x)
+    // with the constraint in global memory, or part(q, x, first lane) with a
+    // lane per component; a sweep that changes impulses stores them.
+    const uint32_t group = lane / 3u, comp = lane % 3u, first = 3u * (group < kLaneCons ? group : 0u);
+    auto sweep = [&](float* p, bool store, auto&& whole, auto&& part) {
+        if (SHARED && chunks) {
+            bring(0u, tid, nt);
+            __syncthreads();
+            for (uint32_t q = 0; q != chunks; ++q) {
+                if (tid >= 32u) {
+                    if (q + 1u < chunks) bring(q + 1u, tid - 32u, nt - 32u);
+                } else {
+                    const TriCon* con = buf[q & 1u];
+                    const uint32_t* st = start[q & 1u];
+                    const uint32_t levels = s_first[q + 1] - s_first[q], base = ls[s_first[q]];
+                    float* pc = p + comp * n;
+                    const uint32_t mine = group < kLaneCons ? group : ~0u >> 1;
+                    auto run = [&](uint32_t j, bool on, LaneCon& x) {
+                        LaneQuad v4 = lane_load(pc, x);
+                        part(v4, x, first, on);
+                        if (on) {
+                            lane_store(pc, x, v4);
+                            if (store) (&s.con[base + j].ni)[comp] = comp == 0u ? x.imp.x : comp == 1u ? x.imp.y : x.imp.z;
+                        }
+                    };
+                    uint32_t j0 = st[0], j1 = st[1];
+                    LaneCon x = lane_con(con + (j0 + mine < j1 ? j0 + mine : j0), comp);
+                    for (uint32_t L = 0; L < levels; ++L) {
+                        // the next level's constraints, while this one's arithmetic runs
+                        const uint32_t k1 = L + 1u < levels ? st[L + 2u] : j1;
+                        const LaneCon y = lane_con(con + (j1 + mine < k1 ? j1 + mine : j0), comp);
+                        run(j0 + mine, j0 + mine < j1, x);
+                        for (uint32_t o = j0 + kLaneCons; o < j1; o += kLaneCons) {  // wide levels
+                            LaneCon w = lane_con(con + (o + mine < j1 ? o + mine : j0), comp);
+                            run(o + mine, o + mine < j1, w);
+                        }
+                        __syncwarp();
+                        x = y;
+                        j0 = j1;
+                        j1 = k1;
+                    }
+                }
+                __syncthreads();
+            }
+        } else if (narrow) {
             if (tid < 32u) {
                 for (uint32_t L = 1; L <= top; ++L) {
                     const uint32_t j = ls[L] + lane;
-                    if (j < ls[L + 1]) fn(j);
+                    if (j < ls[L + 1]) whole(p, s.con[j]);
                     __syncwarp();
                 }
             }
             __syncthreads();
         } else {
             for (uint32_t L = 1; L <= top; ++L) {
-                for (uint32_t j = ls[L] + tid; j < ls[L + 1]; j += nt) fn(j);
+                for (uint32_t j = ls[L] + tid; j < ls[L + 1]; j += nt) whole(p, s.con[j]);
                 __syncthreads();
             }
         }
     };
+    float* v = SHARED ? plane : c.v;
+    if (SHARED) {
+        for (uint32_t i = tid; i < 3u * n; i += nt) plane[i] = c.v[i];
+        __syncthreads();
+    }
 
     // warm start: body contacts, then triangle contacts
     uint32_t body_active = 0;
@@ -556,27 +795,34 @@ __global__ void __launch_bounds__(kSolveThreads) k_sc_solve(ClothDev c, SelfDev 
         int order[kMaxBodyContacts];
         const int k = c.nsph ? body_order(c, i, order) : 0;
         body_active += (uint32_t)k;
-        if (k) body_warm_start(c, i, order, k);
+        if (k) body_warm_start(c, v, i, order, k);
     }
     if (body_active) atomicAdd(&sc->active_contacts, body_active);
     __syncthreads();
-    sweep([&](uint32_t j) { tri_warm_start(c, s.con[s.by_level[j]]); });
+    sweep(v, false, [&](float* p, const TriCon& x) { tri_warm_start(p, n, x); },
+          [&](LaneQuad& q, LaneCon& x, uint32_t, bool) { lane_warm_start(q, x); });
     // velocity iterations
     for (uint32_t it = 0; it < sc->vel_iters; ++it) {
         for (uint32_t i = tid; i < n; i += nt) {
             int order[kMaxBodyContacts];
             const int k = c.nsph ? body_order(c, i, order) : 0;
-            if (k) body_velocity(c, i, order, k);
+            if (k) body_velocity(c, v, i, order, k);
         }
         __syncthreads();
-        sweep([&](uint32_t j) { tri_velocity(c, s.con[s.by_level[j]]); });
+        sweep(v, true, [&](float* p, TriCon& x) { tri_velocity(p, n, x); },
+              [&](LaneQuad& q, LaneCon& x, uint32_t f, bool) { lane_velocity(q, x, f); });
     }
     // store impulses (body impulses live in c_imp already); integrate positions
-    for (uint32_t a = tid; a < A; a += nt) {
-        const TriCon& x = s.con[a];
-        s.imp[cur][s.active_idx[a]] = make_float4(x.ni, x.ti1, x.ti2, 0.0f);
+    for (uint32_t j = tid; j < A; j += nt) {
+        const TriCon& x = s.con[j];
+        s.imp[cur][s.active_idx[s.by_level[j]]] = make_float4(x.ni, x.ti1, x.ti2, 0.0f);
     }
-    for (uint32_t i = tid; i < n; i += nt) st3(c.x, n, i, ld3(c.x, n, i) + h * ld3(c.v, n, i));
+    float* x = SHARED ? plane : c.x;
+    for (uint32_t i = tid; i < n; i += nt) {
+        const f3 vel = ld3(v, n, i), pos = ld3(c.x, n, i) + h * vel;
+        if (SHARED) st3(c.v, n, i, vel);
+        st3(x, n, i, pos);
+    }
     __syncthreads();
     // position iterations with the early out (cloth_solver.cpp:149-164)
     for (uint32_t it = 0; it < sc->pos_iters; ++it) {
@@ -587,16 +833,19 @@ __global__ void __launch_bounds__(kSolveThreads) k_sc_solve(ClothDev c, SelfDev 
             int order[kMaxBodyContacts];
             const int k = c.nsph ? body_order(c, i, order) : 0;
             if (k) {
-                const float ms = body_position(c, i, order, k);
+                const float ms = body_position(c, x, i, order, k);
                 mb = mb < ms ? mb : ms;
             }
         }
         if (mb < 0.0f) atomicMin(&s_min[0], enc_min(mb));
         __syncthreads();
         float mt = 0.0f;
-        sweep([&](uint32_t j) {
-            const float sep = tri_position(c, s.con[s.by_level[j]]);
+        sweep(x, false, [&](float* p, const TriCon& y) {
+            const float sep = tri_position(p, n, y);
             mt = mt < sep ? mt : sep;
+        }, [&](LaneQuad& q, LaneCon& y, uint32_t f, bool on) {
+            const float sep = lane_position(q, y, f);
+            if (on) mt = mt < sep ? mt : sep;
         });
         if (mt < 0.0f) atomicMin(&s_min[1], enc_min(mt));
         __syncthreads();
@@ -604,6 +853,8 @@ __global__ void __launch_bounds__(kSolveThreads) k_sc_solve(ClothDev c, SelfDev 
         __syncthreads();
         if (solved) break;
     }
+    if (SHARED)
+        for (uint32_t i = tid; i < 3u * n; i += nt) c.x[i] = plane[i];
 }
 
 // Triangle proxies after the step (cloth.cpp:580-597): displacement dt times
@@ -893,8 +1144,9 @@ b3g_status self_attach(b3g_cloth* c)
     if (t) k_sc_init_proxies<<<blocks(t, 256), 256, 0, st>>>(c->dev);
     count_launches(t ? 2 : 1);
     SC_TRY(cudaGetLastError());
-    SC_TRY(cudaFuncSetAttribute(k_sc_solve, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    SC_TRY(cudaFuncSetAttribute(k_sc_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)(kSelfMaxParticles * sizeof(uint32_t))));
+    SC_TRY(cudaFuncSetAttribute(k_sc_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSolveSmem));
     SC_TRY(cudaStreamSynchronize(st));
     return B3G_OK;
 }
@@ -929,9 +1181,12 @@ b3g_status self_update(b3g_cloth* c, cudaStream_t st)
 b3g_status self_solve(b3g_cloth* c, cudaStream_t st)
 {
     SelfState* s = c->self;
-    const size_t smem = (size_t)c->dev.n * sizeof(uint32_t);
+    const uint32_t smem = c->dev.n * (uint32_t)sizeof(uint32_t);
     if (c->dev.n > kSelfMaxParticles) return B3G_ERR_UNSUPPORTED;
-    k_sc_solve<<<1, kSolveThreads, smem, st>>>(c->dev, s->d, s->cur);
+    if (c->dev.n <= kSharedParticles)
+        k_sc_solve<true><<<1, kSharedThreads, kSolveSmem, st>>>(c->dev, s->d, s->cur, kSolveSmem);
+    else
+        k_sc_solve<false><<<1, kSolveThreads, smem, st>>>(c->dev, s->d, s->cur, smem);
     count_launches(1);
     SC_TRY(cudaGetLastError());
     return B3G_OK;

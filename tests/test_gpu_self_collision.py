@@ -130,3 +130,40 @@ def test_self_collision_levels_and_limits(b3g):
     with pytest.raises(b3g.B3gError):
         batch.step([gpu], scene.dt)
     batch.close()
+
+
+@pytest.mark.parametrize("side,every", [(14, 1), (40, 3), (91, 3)])
+def test_folded_layers_match_oracle(b3g, port, side, every):
+    """The contact solve's forms: a sheet folded onto itself (few contacts a
+    level, long chains), and layers that touch at every third vertex only (more
+    contacts a level than a warp; 91 x 91 also more particles than the planes
+    in shared memory hold).  From the GPU's state after the contacts were
+    found, one step matches the oracle's as in the tests above."""
+    scene = b3g.self_collision_scene(side)
+    gpu, ora = _pair(b3g, port, scene, b3g.SolverOptions.relative(1e-6, 1000, b3g.DOT_F64))
+    x = scene.mesh.vertices.astype(np.float64)
+    crease = 0.5 * (side % 2)
+    half = np.where(x[:, 0] > crease, 1.0, -1.0)
+    x[:, 1] = 1.6 + 0.5 * (0.37 if every == 1 else 0.55) * half
+    if every > 1:
+        row, col = np.divmod(np.arange(side * side), side)
+        x[(row % every == 1) & (col % every == 1) & (half > 0), 1] -= 0.2
+    x[:, 0] = np.abs(x[:, 0] - crease)
+    rng = np.random.default_rng(side)
+    v = rng.normal(0.0, 0.05, x.shape)
+    v[:, 1] -= 0.5 * half
+    x, v = x.astype(np.float32), v.astype(np.float32)
+    for cloth in (gpu, ora):
+        (cloth.write_state if cloth is gpu else cloth.set_state)(x=x, v=v, dv=np.zeros_like(x))
+    for step in range(2):
+        st = gpu.state()
+        ora.set_state(x=st["x"], v=st["v"], dv=st["dv"])
+        gpu.step(scene.dt)
+        ora.step(scene.dt)
+        gs, os_ = gpu.state(), ora.state()
+        assert rel_err(gs["x"], os_["x"]) <= 1e-4, step
+        assert rel_err(gs["v"], os_["v"]) <= 1e-4, step
+        _compare_lists(gpu.tri_contacts(), ora.tri_contacts(), step)
+    stats = gpu.self_stats()
+    assert stats["active"] > 50
+    assert (stats["active"] > 32 * stats["levels"]) == (every > 1)
