@@ -54,6 +54,23 @@ __device__ __forceinline__ m3 block_at(const ClothDev& c, uint32_t idx)
               f3{v[6 * E + idx], v[7 * E + idx], v[8 * E + idx]}};
 }
 
+// ONCE: a block of a matrix that L2 cannot hold until the next pass; it is
+// marked to leave first, so that the records, which the pass reads about
+// seven times each, stay.  At 1024^2 (k_grid_cg_fused, with the prefetch of
+// SliceAhead in both): 121.7 us an iteration without the mark, 111.9 with it;
+// at 600^2 51.1 and 39.0.  The two-phase form's gathers are half as large and
+// it is slower with the mark (123 and 142 us), so it reads its blocks plainly.
+template <bool ONCE>
+__device__ __forceinline__ m3 block_of(const ClothDev& c, uint32_t idx)
+{
+    if (!ONCE) return block_at(c, idx);
+    const float* v = c.vals;
+    const uint32_t E = c.E;
+    return m3{f3{__ldcs(v + idx), __ldcs(v + E + idx), __ldcs(v + 2 * E + idx)},
+              f3{__ldcs(v + 3 * E + idx), __ldcs(v + 4 * E + idx), __ldcs(v + 5 * E + idx)},
+              f3{__ldcs(v + 6 * E + idx), __ldcs(v + 7 * E + idx), __ldcs(v + 8 * E + idx)}};
+}
+
 // Block k of a thread's row kept in shared memory, [slot][component][thread].
 __device__ __forceinline__ m3 smem_block(const float* sa, uint32_t k, uint32_t B, uint32_t tid)
 {
@@ -264,7 +281,7 @@ __device__ __forceinline__ f3 reg_row_times_direction(const ClothDev& c, const R
 // SMEM_A (one-row form only): the CTA's rows' blocks are copied into shared
 // memory at the start, [slot][component][thread], and every later product
 // reads them there; only the neighbours' z and p come from L2.
-template <int DOT, bool ONE_ROW, bool SMEM_A>
+template <int DOT, bool ONE_ROW, bool SMEM_A, bool STREAM = false>
 __global__ void __launch_bounds__(kMaxBlock) k_grid_cg(const __grid_constant__ ClothDev c, GridBarrier* bar)
 {
     extern __shared__ float smem_a[];
@@ -362,7 +379,9 @@ __global__ void __launch_bounds__(kMaxBlock) k_grid_cg(const __grid_constant__ C
                     v1[0] = D::add_term(v1[0], p, s);
                 }
             } else {
+                SliceAhead<STREAM> ahead(c, first_row >> 5, stride >> 5);
                 for (uint32_t row = first_row; row < n; row += stride) {
+                    ahead.next(c);
                     const f3 zi = ld3(c.z, n, row);
                     const f3 pr = first ? zi : zi + beta * ld3(pold, n, row);
                     const f3 ap = row_times_direction(c, row, c.z, pold, beta, first);
@@ -430,9 +449,10 @@ timeout:
 }
 
 template <int DOT>
-const void* grid_kernel(bool one_row, bool smem_a)
+const void* grid_kernel(bool one_row, bool smem_a, bool stream)
 {
-    if (!one_row) return (const void*)k_grid_cg<DOT, false, false>;
+    if (!one_row)
+        return stream ? (const void*)k_grid_cg<DOT, false, false, true> : (const void*)k_grid_cg<DOT, false, false>;
     return smem_a ? (const void*)k_grid_cg<DOT, true, true> : (const void*)k_grid_cg<DOT, true, false>;
 }
 
@@ -605,7 +625,7 @@ __device__ __forceinline__ bool fused_scalars(const StepScalars* sc, double ps, 
 // SMEM_A (one-row form only): the CTA's rows' blocks are copied into shared
 // memory at the start, [slot][component][thread], and every later product
 // reads them there; only the neighbours' records come from L2.
-template <int DOT, bool ONE_ROW, bool SMEM_A>
+template <int DOT, bool ONE_ROW, bool SMEM_A, bool STREAM = false>
 __global__ void __launch_bounds__(kMaxBlock) k_grid_cg_fused(const __grid_constant__ ClothDev c, GridBarrier* bar,
                                                              float4* rec0, float4* rec1)
 {
@@ -722,7 +742,11 @@ __global__ void __launch_bounds__(kMaxBlock) k_grid_cg_fused(const __grid_consta
                     F::add(v4[0], p, s, z, r, sp);
                 }
             } else {
+                SliceAhead<STREAM> ahead(c, first_row >> 5, stride >> 5);
                 for (uint32_t row = first_row; row < n; row += stride) {
+                    if (STREAM && (threadIdx.x & 31u) == 10u && ahead.len && 32u * ahead.q + 32u <= n)
+                        prefetch_l2(rin + 96 * (size_t)ahead.q, 1536u);  // a full slice's records
+                    ahead.next(c);
                     const Rec own = ld_rec(rin, row);
                     f3 rv = own.r, pv;
                     if (!first) {
@@ -733,7 +757,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_grid_cg_fused(const __grid_consta
                     pv = first ? z : z + beta * own.p;
                     const uint32_t base = rbase(c, row);
                     const uint32_t deg = c.row_deg[row];
-                    f3 acc = zero3() + block_at(c, base) * pv;
+                    f3 acc = zero3() + block_of<STREAM>(c, base) * pv;
                     constexpr int W = 4;
                     for (uint32_t k0 = 1; k0 < deg; k0 += W) {
                         uint32_t cl[W];
@@ -742,7 +766,7 @@ __global__ void __launch_bounds__(kMaxBlock) k_grid_cg_fused(const __grid_consta
 #pragma unroll
                         for (int k = 0; k < W; ++k) {
                             if (k0 + k < deg) {
-                                const m3 a = block_at(c, base + 32u * (k0 + k));
+                                const m3 a = block_of<STREAM>(c, base + 32u * (k0 + k));
                                 const Rec q = ld_rec(rin, cl[k]);
                                 acc = acc + a * rec_direction(q, alpha, beta, first);
                             }
@@ -799,11 +823,22 @@ timeout:
 }
 
 template <int DOT>
-const void* fused_kernel(bool one_row, bool smem_a)
+const void* fused_kernel(bool one_row, bool smem_a, bool stream)
 {
-    if (!one_row) return (const void*)k_grid_cg_fused<DOT, false, false>;
+    if (!one_row)
+        return stream ? (const void*)k_grid_cg_fused<DOT, false, false, true>
+                      : (const void*)k_grid_cg_fused<DOT, false, false>;
     return smem_a ? (const void*)k_grid_cg_fused<DOT, true, true> : (const void*)k_grid_cg_fused<DOT, true, false>;
 }
+
+// Whether a cloth's matrix (36 bytes a block and 4 of its column) is too large
+// to stay in L2 between two passes beside the vectors: the STREAM form.  Without
+// and with it, us an iteration: one-pass form 37.0 and 29.2 at 520^2 (76 MB and
+// 25 MB of records), 50.1 and 39.2 at 600^2, 130 and 110.7 at 1024^2 (294 MB);
+// below 70 MiB level or slower (450^2: 21.1 and 22.8).  Two-phase form, which
+// reads less beside the matrix: 25.7 and 26.9 at 480^2, 36.3 and 36.9 at 520^2,
+// 54.7 and 50.6 at 600^2 (101 MB), 146 and 120.8 at 1024^2.
+bool streamed(const ClothDev& c, bool fused) { return 40ull * c.E > (fused ? 70ull << 20 : 84ull << 20); }
 
 }  // namespace
 
@@ -819,11 +854,14 @@ GridCgShape grid_cg_shape(uint32_t n, int device, bool fused)
         g.blocks = (int)((n + g.threads - 1) / g.threads);
     } else {
         int per_sm = 1;
-        const void* fn = fused ? (const void*)k_grid_cg_fused<2, false, false> : (const void*)k_grid_cg<2, false, false>;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kMaxBlock, 0) != cudaSuccess ||
-            per_sm < 1) {
-            cudaGetLastError();
-            per_sm = 1;
+        for (bool stream : {false, true}) {  // the same grid, and so the same order of sums, for both
+            const void* fn = fused ? fused_kernel<2>(false, false, stream) : grid_kernel<2>(false, false, stream);
+            int fit = 1;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, kMaxBlock, 0) != cudaSuccess || fit < 1) {
+                cudaGetLastError();
+                fit = 1;
+            }
+            per_sm = stream ? std::min(per_sm, fit) : fit;
         }
         g.threads = kMaxBlock;
         g.blocks = std::min(sms * per_sm, kMaxGridCgBlocks);
@@ -851,8 +889,9 @@ cudaError_t launch_grid_cg(const ClothDev& c, int dot, GridBarrier* bar, cudaStr
     // shared memory of the reductions
     const size_t smem = (size_t)c.max_deg * 9 * sizeof(float) * (size_t)g.threads;
     const bool smem_a = one_row && smem + 4096 <= kSmemLimit;
-    const void* fn = dot == 2 ? grid_kernel<2>(one_row, smem_a)
-                   : dot == 1 ? grid_kernel<1>(one_row, smem_a) : grid_kernel<0>(one_row, smem_a);
+    const bool stream = streamed(c, false);
+    const void* fn = dot == 2 ? grid_kernel<2>(one_row, smem_a, stream)
+                   : dot == 1 ? grid_kernel<1>(one_row, smem_a, stream) : grid_kernel<0>(one_row, smem_a, stream);
     if (smem_a) {
         cudaError_t ea = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (ea != cudaSuccess) return ea;
@@ -883,8 +922,9 @@ cudaError_t launch_grid_cg_fused(const ClothDev& c, int dot, GridBarrier* bar, f
     // shared memory of the reductions
     const size_t smem = (size_t)c.max_deg * 9 * sizeof(float) * (size_t)g.threads;
     const bool smem_a = one_row && smem + 4096 <= kSmemLimit;
-    const void* fn = dot == 2 ? fused_kernel<2>(one_row, smem_a)
-                   : dot == 1 ? fused_kernel<1>(one_row, smem_a) : fused_kernel<0>(one_row, smem_a);
+    const bool stream = streamed(c, true);
+    const void* fn = dot == 2 ? fused_kernel<2>(one_row, smem_a, stream)
+                   : dot == 1 ? fused_kernel<1>(one_row, smem_a, stream) : fused_kernel<0>(one_row, smem_a, stream);
     if (smem_a) {
         cudaError_t ea = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (ea != cudaSuccess) return ea;

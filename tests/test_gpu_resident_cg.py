@@ -47,6 +47,29 @@ def test_on_chip_cg_matches_launches(b3g, kind, side, dot):
     assert np.abs(a - b).max() <= (1e-6 if dot == 2 else 1e-5) * np.abs(a).max()
 
 
+@pytest.mark.parametrize("kind,side", [("plain", 517), ("plain", 577), ("bend", 450)])
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("dot", [0, 2])
+def test_streamed_matrix_matches_launches(b3g, kind, side, fused, dot):
+    """Cloths whose matrix does not stay in L2 (a last slice that is not full;
+    rows with and without bending), with the same bound; the one-pass form
+    rounds beta's numerator apart, one more rounding an iteration."""
+    scene = _scene(b3g, kind, side)
+    opts = b3g.SolverOptions(b3g.STOP_RELATIVE, 1e-9, 8, dot)
+    rng = np.random.default_rng(side)
+    v = rng.normal(0.0, 0.1, (scene.mesh.vertex_count, 3)).astype(np.float32)
+    v[np.asarray(scene.pinned, np.int64)] = 0.0
+    got = []
+    for persistent in (False, True):
+        cloth = b3g.Cloth(scene.mesh, scene.cdef).setup(scene, opts)
+        cloth.set_cg_strategy(persistent, fused and persistent)
+        cloth.write_state(v=v, dv=0.1 * v)
+        cloth.step(scene.dt)
+        got.append(cloth.state()["dv"].astype(np.float64))
+        cloth.close()
+    assert np.abs(got[0] - got[1]).max() <= 1e-5 * np.abs(got[0]).max()
+
+
 def test_on_chip_cg_repeats_itself(b3g):
     """The grid form's sums run in a fixed order: the same step twice gives the
     same bits."""
