@@ -1908,6 +1908,11 @@ b3g_status b3g_cloth_read_state(const b3g_cloth* cc, float* x, float* v, float* 
     cudaSetDevice(c->device);
     b3g_status s = flush_ops(c);
     if (s != B3G_OK) return s;
+    const uint32_t n = c->dev.n;
+    bool taken = false;
+    B3G_TRY(host_stage_copy({{c->dev.x, x, 3 * n, n}, {c->dev.v, v, 3 * n, n}, {c->dev.mx, mx, 3 * n, n}},
+                            true, c->stream, &taken));
+    if (taken) return B3G_OK;
     if (x && (s = read_planes(c, c->dev.x, x)) != B3G_OK) return s;
     if (v && (s = read_planes(c, c->dev.v, v)) != B3G_OK) return s;
     if (mx && (s = read_planes(c, c->dev.mx, mx)) != B3G_OK) return s;
@@ -1923,6 +1928,12 @@ b3g_status b3g_cloth_write_state(b3g_cloth* c, const float* x, const float* v, c
     const uint32_t n = c->dev.n;
     const float* srcs[3] = {x, v, mx};
     float* dsts[3] = {c->dev.x, c->dev.v, c->dev.mx};
+    bool taken = false;
+    B3G_TRY(host_stage_copy({{dsts[0], const_cast<float*>(x), 3 * n, n},
+                             {dsts[1], const_cast<float*>(v), 3 * n, n},
+                             {dsts[2], const_cast<float*>(mx), 3 * n, n}},
+                            false, c->stream, &taken));
+    if (taken) return B3G_OK;
     for (int k = 0; k < 3; ++k) {
         if (!srcs[k]) continue;
         B3G_TRY(cudaMemcpyAsync(c->d_stage, srcs[k], 3 * (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));

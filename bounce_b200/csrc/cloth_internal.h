@@ -6,6 +6,7 @@
 #include <vector>
 
 #include "../../include/b3g.h"
+#include "host_stage.h"
 #include "cloth_dev.cuh"
 #include "topology.h"
 
@@ -63,6 +64,7 @@ struct b3g_cloth {
     bool row_assembly = false;  // the row-centric assembly even where the slot-major one applies
     bool lean_layout = false;   // laid out without the slot-major assembly's records (server cloths)
 
+    b3g::HostStageUse stage_use;  // read_state and write_state
     // pinned staging
     b3g::StepScalars* h_sc = nullptr;
     b3g::ParticleOp* h_ops = nullptr;

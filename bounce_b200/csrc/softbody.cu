@@ -29,6 +29,7 @@
 #include "../../include/b3g.h"
 #include "cloth_dev.cuh"
 #include "grid_cg.cuh"
+#include "host_stage.h"
 #include "mpcg_solve.cuh"
 #include "resident_cg.h"
 #include "hull_gjk.cuh"
@@ -815,6 +816,7 @@ using namespace b3g;
 struct b3g_softbody {
     int device = 0;
     cudaStream_t stream = nullptr;
+    HostStageUse stage_use;  // the state and element transfers
     char* arena = nullptr;
     SoftDev dev{};
     CsrSystem cs{};
@@ -1339,6 +1341,11 @@ b3g_status b3g_softbody_step(b3g_softbody* b, float dt, uint32_t velocity_iterat
     return h.status ? (b3g_status)h.status : B3G_OK;
 }
 
+static StageArray node_words(float* dev, const float* host, uint32_t words)
+{
+    return StageArray{dev, const_cast<float*>(host), words, 0u};
+}
+
 static b3g_status copy_nodes(b3g_softbody* b, float* dst, const float* src, size_t bytes, cudaMemcpyKind kind)
 {
     SB_TRY(cudaMemcpyAsync(dst, src, bytes, kind, b->stream));
@@ -1456,6 +1463,11 @@ b3g_status b3g_softbody_read_state(const b3g_softbody* cb, float* x, float* v)
     if (!ok(b)) return B3G_ERR_INVALID_ARGUMENT;
     cudaSetDevice(b->device);
     const size_t vec = 3 * (size_t)b->dev.n * sizeof(float);
+    bool taken = false;
+    SB_TRY(host_stage_copy({node_words(b->dev.x, x, 3 * b->dev.n),
+                            node_words(b->dev.v, v, 3 * b->dev.n)},
+                           true, b->stream, &taken));
+    if (taken) return B3G_OK;
     b3g_status r = B3G_OK;
     if (x && (r = copy_nodes(b, x, b->dev.x, vec, cudaMemcpyDeviceToHost)) != B3G_OK) return r;
     if (v && (r = copy_nodes(b, v, b->dev.v, vec, cudaMemcpyDeviceToHost)) != B3G_OK) return r;
@@ -1467,6 +1479,11 @@ b3g_status b3g_softbody_write_state(b3g_softbody* b, const float* x, const float
     if (!ok(b)) return B3G_ERR_INVALID_ARGUMENT;
     cudaSetDevice(b->device);
     const size_t vec = 3 * (size_t)b->dev.n * sizeof(float);
+    bool taken = false;
+    SB_TRY(host_stage_copy({node_words(b->dev.x, x, 3 * b->dev.n),
+                            node_words(b->dev.v, v, 3 * b->dev.n)},
+                           false, b->stream, &taken));
+    if (taken) return B3G_OK;
     b3g_status r = B3G_OK;
     if (x && (r = copy_nodes(b, b->dev.x, x, vec, cudaMemcpyHostToDevice)) != B3G_OK) return r;
     if (v && (r = copy_nodes(b, b->dev.v, v, vec, cudaMemcpyHostToDevice)) != B3G_OK) return r;
@@ -1478,6 +1495,11 @@ b3g_status b3g_softbody_read_elements(const b3g_softbody* cb, float* q, float* e
     b3g_softbody* b = const_cast<b3g_softbody*>(cb);
     if (!ok(b)) return B3G_ERR_INVALID_ARGUMENT;
     cudaSetDevice(b->device);
+    bool taken = false;
+    SB_TRY(host_stage_copy({node_words((float*)b->dev.q, q, 4 * b->dev.t),
+                            node_words(b->dev.eps, eps, 6 * b->dev.t)},
+                           true, b->stream, &taken));
+    if (taken) return B3G_OK;
     b3g_status r = B3G_OK;
     if (q && (r = copy_nodes(b, q, (const float*)b->dev.q, (size_t)b->dev.t * 16, cudaMemcpyDeviceToHost)) != B3G_OK)
         return r;
@@ -1489,6 +1511,11 @@ b3g_status b3g_softbody_write_elements(b3g_softbody* b, const float* q, const fl
 {
     if (!ok(b)) return B3G_ERR_INVALID_ARGUMENT;
     cudaSetDevice(b->device);
+    bool taken = false;
+    SB_TRY(host_stage_copy({node_words((float*)b->dev.q, q, 4 * b->dev.t),
+                            node_words(b->dev.eps, eps, 6 * b->dev.t)},
+                           false, b->stream, &taken));
+    if (taken) return B3G_OK;
     b3g_status r = B3G_OK;
     if (q && (r = copy_nodes(b, (float*)b->dev.q, q, (size_t)b->dev.t * 16, cudaMemcpyHostToDevice)) != B3G_OK) return r;
     if (eps && (r = copy_nodes(b, b->dev.eps, eps, (size_t)b->dev.t * 24, cudaMemcpyHostToDevice)) != B3G_OK) return r;
