@@ -65,7 +65,8 @@ uint32_t resident_chunk(uint32_t n, bool grid);
 
 // Fills c.halo_team and c.halo_grid where the band is too wide for the
 // threads of a CTA: the most rows outside a CTA's chunk that its rows touch.
-// each(i, f): f(column) for every column of row i.
+// each(i, f): f(column) for every column of row i.  Counting ends where a CTA
+// already touches more than the threads of any shape hold.
 template <class Each>
 void resident_halos(ClothDev& c, Each&& each)
 {
@@ -75,9 +76,10 @@ void resident_halos(ClothDev& c, Each&& each)
         if (!chunk || !res_wide(n, chunk, c.band, kResMaxThreads)) continue;
         std::vector<uint32_t> seen(n, ~0u);
         uint32_t most = 0;
-        for (uint32_t r0 = 0; r0 < n; r0 += chunk) {
+        const uint32_t bound = kResHalo * kResMaxThreads;
+        for (uint32_t r0 = 0; r0 < n && most <= bound; r0 += chunk) {
             uint32_t count = 0;
-            for (uint32_t i = r0; i < r0 + chunk && i < n; ++i)
+            for (uint32_t i = r0; i < r0 + chunk && i < n && count <= bound; ++i)
                 each(i, [&](uint32_t j) {
                     if (j - r0 >= chunk && seen[j] != r0) seen[j] = r0, ++count;
                 });
