@@ -25,6 +25,7 @@ __global__ void __launch_bounds__(kResMaxThreads, 1)
     team.zs = reinterpret_cast<float*>(smem + kResHeader) + 3u * (size_t)res_rows(c.n, chunk, c.band, listed);
     uint32_t phase = 0u;
     res_init_copy_barrier(sh);
+    team.barrier();  // every CTA runs before another writes into it
     resident_solve<DOT, RPT, SLOTS>(c, team, smem, chunk, listed, smem_bytes, phase);
     team.barrier();  // no CTA leaves while another may still write into it
 }
