@@ -94,16 +94,9 @@ const void* kernel_for(int dot)
 
 }  // namespace
 
-// A window of more than half of the shared memory leaves too little for the
-// blocks; more than one row a thread is for rows of up to
-// kResFewSlots blocks.
 bool batch_on_chip(const ClothDev& c, int team)
 {
-    const uint32_t slices = (c.n + 31u) / 32u, per = (slices + (uint32_t)team - 1u) / (uint32_t)team;
-    if (per > (uint32_t)(kResBatchRows * kResMaxWarps)) return false;
-    if (c.max_deg > (uint32_t)(per > (uint32_t)kResMaxWarps ? kResFewSlots : kResSlots)) return false;
-    return !res_wide(c.n, 32u * per, c.band, kResMaxThreads) &&
-           res_block_offset(res_window(c.n, 32u * per, c.band), 12u * 32u * per) <= kResSmemLimit / 2u;
+    return resident_in_batch({c.n, c.E, c.max_deg, c.band, 0u, 0u}, (uint32_t)team);
 }
 
 cudaError_t launch_batch_resident(const BatchCgArgs& a, int team, int dot, cudaStream_t st)

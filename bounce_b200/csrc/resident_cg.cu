@@ -1,8 +1,6 @@
 // Launches of the on-chip MPCG (resident_cg.cuh) for one cloth.
 #include "resident_cg.h"
 
-#include <algorithm>
-
 #include "resident_cg.cuh"
 
 namespace b3g {
@@ -78,65 +76,12 @@ const void* kernel_for(bool grid, uint32_t rpt, uint32_t deg)
 
 }  // namespace
 
-uint32_t resident_team(uint32_t n)
-{
-    if (n > (uint32_t)(kResMaxTeam * kResMaxThreads)) return 0u;
-    uint32_t t = 1;
-    while (n > 256u && t < (uint32_t)kResMaxTeam && n > t * 128u) t *= 2;
-    return t;
-}
-
-uint32_t resident_chunk(uint32_t n, bool grid)
-{
-    const uint32_t slices = (n + 31u) / 32u, ctas = grid ? 148u : resident_team(n);
-    return ctas ? 32u * ((slices + ctas - 1u) / ctas) : 0u;
-}
-
 ResShape resident_shape(const ClothDev& c)
 {
-    ResShape s;
-    if (c.max_deg > (uint32_t)kResWideSlots || c.n == 0) return s;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const uint32_t n = c.n, slices = (n + 31u) / 32u;
-    auto shape = [&](bool grid, uint32_t ctas) {
-        ResShape r;
-        const uint32_t per = (slices + ctas - 1u) / ctas, most = (uint32_t)kResMaxThreads;
-        r.grid = grid;
-        r.chunk = 32u * per;
-        r.ctas = grid ? (n + r.chunk - 1u) / r.chunk : ctas;
-        r.rows_per_thread = r.chunk <= most ? 1u : 2u;
-        const uint32_t own = 32u * ((per + r.rows_per_thread - 1u) / r.rows_per_thread);
-        // threads without rows of their own help with the halo
-        const bool wide = res_wide(n, r.chunk, c.band, most);
-        if (wide && r.chunk == resident_chunk(n, grid)) r.listed = grid ? c.halo_grid : c.halo_team;
-        const uint32_t halo = wide ? r.listed : res_window(n, r.chunk, c.band) - std::min(n, r.chunk);
-        r.threads = std::max(own, 32u * ((halo + 32u * kResHalo - 1u) / (32u * kResHalo)));
-        if (grid) r.threads = std::max(r.threads, 32u * ((r.ctas + 31u) / 32u));  // a thread a partial
-        const uint64_t off = res_block_offset(res_rows(n, r.chunk, c.band, r.listed),
-                                              !grid && ctas > 1u ? 12u * r.chunk : 0u);
-        // (listing needs two words a 32 rows and one a halo row beside the window)
-        const uint64_t all = off + std::max<uint64_t>((uint64_t)r.chunk * c.max_deg * 36u,
-                                            r.listed ? 8ull * slices + 4ull * r.listed : 0ull);
-        r.smem = (uint32_t)std::min<uint64_t>(all, kResSmemLimit);
-        if ((wide && !r.listed) || r.threads > most) r.ctas = 0;
-        // at least half of the blocks resident, on average
-        if (off + (uint64_t)per * (c.E / slices) * 18u > kResSmemLimit) r.ctas = 0;
-        if (r.listed && off + 8ull * slices + 4ull * r.listed > kResSmemLimit) r.ctas = 0;
-        if (r.rows_per_thread > 1u && c.max_deg > (uint32_t)kResSlots) r.ctas = 0;
-        return r;
-    };
-    // One CTA to 256 rows, then clusters of up to 8 CTAs of 128 to 512 rows,
-    // then the grid.  Measured per iteration (FP64 dots, 7 blocks a row): 256
-    // rows 2.6 us on one CTA and 2.9 on two; 1,024 rows 3.3 on eight CTAs, 4.2
-    // on two; 4,096 rows 4.5 on eight and 6.2 on the grid; 8,281 rows (13
-    // blocks) 8.5 on a cluster of 16 and 5.4 on the grid.
-    if (const uint32_t t = resident_team(n)) {
-        s = shape(false, t);
-        if (s.ctas) return s;
-    }
-    return shape(true, (uint32_t)std::min(sms, kResMaxGrid));
+    return resident_shape_on({c.n, c.E, c.max_deg, c.band, c.halo_team, c.halo_grid}, sms);
 }
 
 cudaError_t launch_resident_cg(const ClothDev& c, const ResShape& s, int dot, bool by_blocks, cudaStream_t st)

@@ -45,7 +45,6 @@ namespace {
 
 namespace rcg = cooperative_groups;
 
-constexpr int kResMaxWarps = kResMaxThreads / 32;
 constexpr uint32_t kResSpinLimit = 1u << 24;
 constexpr uint32_t kResTimeout = 7;  // B3G_ERR_TIMEOUT
 
