@@ -920,13 +920,13 @@ b3g_status ensure_sell(b3g_softbody* b)
     uint8_t* d_type = (uint8_t*)take(n);
     b->rec = (float4*)take(grid_cg_fused_rec_bytes(n));
     cudaStream_t s = b->stream;
+    // all of it: the on-chip CG knows a row of z that lies in the planes by its
+    // tag alone, and memory that another body gave back may hold the same tags
+    SB_TRY(cudaMemsetAsync(b->pcg, 0, bytes, s));
     SB_TRY(cudaMemcpyAsync(d_inv, inv.data(), (size_t)n * 4, cudaMemcpyHostToDevice, s));
     SB_TRY(cudaMemcpyAsync(d_off, off.data(), (nslices + 1) * 4, cudaMemcpyHostToDevice, s));
     SB_TRY(cudaMemcpyAsync(d_deg, deg.data(), n, cudaMemcpyHostToDevice, s));
     SB_TRY(cudaMemcpyAsync(d_cols, cols.data(), (size_t)E * 4, cudaMemcpyHostToDevice, s));
-    SB_TRY(cudaMemsetAsync(d_vals, 0, (size_t)E * 36, s));
-    SB_TRY(cudaMemsetAsync(partials, 0, kGridCgPartialBytes, s));
-    SB_TRY(cudaMemsetAsync(bar, 0, sizeof(GridBarrier), s));
     SB_TRY(cudaStreamSynchronize(s));  // the host vectors go out of scope
     SoftDev& d = b->dev;
     d.sell_vals = d_vals;
