@@ -1821,31 +1821,36 @@ b3g_status b3g_debug_cg_barrier_timeout(b3g_cloth* c, uint32_t spin_limit, b3g_s
     if (!valid(c) || !c->owns_stream || !result || spin_limit == 0) return B3G_ERR_INVALID_ARGUMENT;
     cudaSetDevice(c->device);
     cudaStream_t st = c->stream;
-    // a barrier that cannot complete: the arrival counter starts half its
-    // range away from every target (the on-chip CG publishes no partials when
-    // it is not zero), so every CTA waits until its limit
-    GridBarrier bar = {0x80000000u, 0u, spin_limit, 0u};
+    // a barrier that cannot complete, so that every CTA waits until its limit:
+    // the arrival counter starts half its range away from every target.  The
+    // on-chip CG publishes nothing when it finds that, and in a second run
+    // everything but its rows of z.  (A cloth solved by one cluster waits on
+    // hardware barriers only: it takes the counter kernel.)
+    const ResShape shape = resident_shape(c->dev);
+    const bool fused = c->cg_strategy == B3G_CG_PERSISTENT_FUSED;
+    const bool resident = !fused && shape.ctas && shape.grid;
     StepScalars* h = c->h_sc;
-    B3G_TRY(cudaStreamSynchronize(st));
-    fill_step_scalars(c, 1.0f / 60.0f, 8, 2, h);
-    c->step_index -= 1;
-    B3G_TRY(cudaMemcpyAsync(c->dev.sc, h, sizeof(StepScalars), cudaMemcpyHostToDevice, st));
-    B3G_TRY(cudaMemcpyAsync(c->dev.bar, &bar, kBarrierClear, cudaMemcpyHostToDevice, st));
-    B3G_TRY(launch_assemble(c->dev, c->assemble_block, st));
-    if (c->cg_strategy == B3G_CG_PERSISTENT_FUSED) {
+    if (fused) {
         b3g_status s = ensure_cg_rec(c);
         if (s != B3G_OK) return s;
-        B3G_TRY(launch_grid_cg_fused(c->dev, (int)c->opts.dot, c->dev.bar, c->cg_rec, st));
-    } else {
-        // (a cloth solved by one cluster waits on hardware barriers only)
-        const ResShape shape = resident_shape(c->dev);
-        B3G_TRY(shape.ctas && shape.grid ? launch_resident_cg(c->dev, shape, (int)c->opts.dot, false, st)
-                                         : launch_grid_cg(c->dev, (int)c->opts.dot, c->dev.bar, st));
     }
-    B3G_TRY(cudaMemsetAsync(c->dev.bar, 0, kBarrierReset, st));
-    B3G_TRY(cudaMemcpyAsync(h, c->dev.sc, sizeof(StepScalars), cudaMemcpyDeviceToHost, st));
-    B3G_TRY(cudaStreamSynchronize(st));
-    *result = (b3g_status)h->status;
+    for (const uint32_t count : {kResWithholdAll, kResWithholdRows}) {
+        const GridBarrier bar = {count, 0u, spin_limit, 0u};
+        B3G_TRY(cudaStreamSynchronize(st));
+        fill_step_scalars(c, 1.0f / 60.0f, 8, 2, h);
+        c->step_index -= 1;
+        B3G_TRY(cudaMemcpyAsync(c->dev.sc, h, sizeof(StepScalars), cudaMemcpyHostToDevice, st));
+        B3G_TRY(cudaMemcpyAsync(c->dev.bar, &bar, kBarrierClear, cudaMemcpyHostToDevice, st));
+        B3G_TRY(launch_assemble(c->dev, c->assemble_block, st));
+        B3G_TRY(resident ? launch_resident_cg(c->dev, shape, (int)c->opts.dot, false, st)
+                : fused  ? launch_grid_cg_fused(c->dev, (int)c->opts.dot, c->dev.bar, c->cg_rec, st)
+                         : launch_grid_cg(c->dev, (int)c->opts.dot, c->dev.bar, st));
+        B3G_TRY(cudaMemsetAsync(c->dev.bar, 0, kBarrierReset, st));
+        B3G_TRY(cudaMemcpyAsync(h, c->dev.sc, sizeof(StepScalars), cudaMemcpyDeviceToHost, st));
+        B3G_TRY(cudaStreamSynchronize(st));
+        *result = (b3g_status)h->status;
+        if (!resident || *result != B3G_ERR_TIMEOUT) break;
+    }
     return B3G_OK;
 }
 

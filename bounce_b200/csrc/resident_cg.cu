@@ -42,7 +42,10 @@ __global__ void __launch_bounds__(kResMaxThreads, 1)
     team.bar = c.bar;
     team.part = reinterpret_cast<ulonglong2*>(static_cast<char*>(c.partials) + kGridCgCounterBytes);
     team.base = *(volatile uint32_t*)&c.bar->nonce;
-    team.mute = *(volatile uint32_t*)&c.bar->count != 0u;
+    const uint32_t withheld = *(volatile uint32_t*)&c.bar->count;
+    team.mute = withheld == kResWithholdAll;
+    team.mute_rows = withheld != 0u;
+    team.row_lost = false;
     team.limit = c.bar->spin_limit ? c.bar->spin_limit : kResSpinLimit;
     team.zt = reinterpret_cast<float4*>(c.p);  // p and s, 6 n floats, are free here
     team.arrivals = *(volatile uint32_t*)&c.bar->arrivals;

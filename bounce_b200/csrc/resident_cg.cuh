@@ -210,7 +210,8 @@ struct GridScope {
     ulonglong2* part;  // [parity][value][rank], a line each
     float4* zt;        // z of every row and a tag of the reduction that follows it
     uint32_t limit;
-    bool mute;         // the diagnostic of the bounded waits: nothing is published
+    bool mute, mute_rows;  // the diagnostic of the bounded waits: nothing, or no row of z, is published
+    bool row_lost;         // this thread gave up on a row
 
     static __device__ void put(ulonglong2* p, unsigned long long v, unsigned long long tag)
     {
@@ -234,19 +235,24 @@ struct GridScope {
     __device__ uint32_t z_tag() const { return 0xffc00000u | ((base + epoch) & 0x3fffffu); }
     __device__ void put_z(const ClothDev&, uint32_t row, uint32_t, uint32_t, f3 z) const
     {
-        if (mute) return;
+        if (mute_rows) return;
         put(reinterpret_cast<ulonglong2*>(zt + row),
             (unsigned long long)__float_as_uint(z.x) | ((unsigned long long)__float_as_uint(z.y) << 32),
             (unsigned long long)__float_as_uint(z.z) | ((unsigned long long)z_tag() << 32));
     }
-    // Row `row` as published under `tag`; the wait is bounded.
-    __device__ f3 get_z(const ClothDev&, uint32_t row, uint32_t, uint32_t tag) const
+    // Row `row` as published under `tag`; the wait is bounded.  Giving up shows in
+    // the next reduction: at once, another thread still at the end of the last
+    // one might see it there and leave the block's barriers by itself.
+    __device__ f3 get_z(const ClothDev&, uint32_t row, uint32_t, uint32_t tag)
     {
         unsigned long long a, b;
         for (uint32_t spins = 0;; ++spins) {
             get(reinterpret_cast<const ulonglong2*>(zt + row), a, b);
             if ((uint32_t)(b >> 32) == tag) break;
-            if (give_up(spins)) break;
+            if (out_of_time(spins)) {
+                row_lost = true;
+                break;
+            }
         }
         return f3{__uint_as_float((uint32_t)a), __uint_as_float((uint32_t)(a >> 32)), __uint_as_float((uint32_t)b)};
     }
@@ -287,11 +293,17 @@ struct GridScope {
             put(part + (((epoch & 1u) * 2u + lane) * kResMaxGrid + rank) * kResLine, pack8(a), base + epoch);
         }
     }
-    __device__ bool give_up(uint32_t spins) const
+    __device__ bool out_of_time(uint32_t spins) const
     {
         if (spins <= limit && ((spins & 63u) != 63u || !failed())) return false;
-        sh->lost = 1;
         fail();
+        return true;
+    }
+    // For the waits that a block barrier follows before anyone reads `lost`.
+    __device__ bool give_up(uint32_t spins) const
+    {
+        if (!out_of_time(spins)) return false;
+        sh->lost = 1;
         return true;
     }
     template <class D, int NV>
@@ -300,6 +312,7 @@ struct GridScope {
         typedef typename D::T T;
         const uint32_t lane = threadIdx.x & 31u;
         double* w = &sh->wsum[0][0][0] + 2 * kResMaxWarps;  // [value][rank]
+        if (row_lost) sh->lost = 1;
         if (threadIdx.x == 0) {
             const uint32_t target = arrivals + epoch * size;
             for (uint32_t spins = 0;; ++spins) {

@@ -32,6 +32,9 @@ constexpr int kResHalo = 4;       // halo rows a thread
 constexpr uint32_t kResHeader = 4736;
 constexpr uint32_t kResBatchStatic = 2048;  // static shared memory of the batch's kernel
 constexpr uint32_t kResSmemLimit = 227 * 1024;
+// GridBarrier::count of a launch that withholds what others wait for (the
+// diagnostic of the bounded waits): everything, or the rows of z.
+constexpr uint32_t kResWithholdAll = 0x80000000u, kResWithholdRows = 1u;
 // Bytes of a grid's tagged partials: two alternating sets of two sums.
 constexpr size_t kResPartialBytes = (size_t)2 * 2 * kResMaxGrid * kResLine * 16;
 

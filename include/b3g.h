@@ -310,7 +310,8 @@ typedef enum { B3G_ASSEMBLY_ELEMENT_RECORDS = 0, B3G_ASSEMBLY_ROWS = 1 } b3g_ass
 b3g_status b3g_cloth_set_assembly(b3g_cloth* cloth, b3g_assembly form);
 b3g_assembly b3g_cloth_get_assembly(const b3g_cloth* cloth);
 /* Diagnostic of the bounded waits: runs the persistent CG once with a grid
- * barrier that can never complete and a wait limit of spin_limit polls;
+ * barrier that can never complete and a wait limit of spin_limit polls (the
+ * on-chip form once more with only its published vectors withheld);
  * *result receives the solve status (B3G_ERR_TIMEOUT when the limit works).
  * The cloth's state is not changed. */
 b3g_status b3g_debug_cg_barrier_timeout(b3g_cloth* cloth, uint32_t spin_limit, b3g_status* result);

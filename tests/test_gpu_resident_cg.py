@@ -113,3 +113,24 @@ def test_batch_on_chip_matches_launches(b3g, cluster, split, dot):
         a.step(scenes[0].dt)
         x, y = a.state()["dv"].astype(np.float64), b.state()["dv"].astype(np.float64)
         assert np.abs(x - y).max() <= (1e-6 if dot == 2 else 1e-5) * np.abs(x).max()
+
+
+@pytest.mark.parametrize("side", [91, 280])
+def test_withheld_rows_time_out(b3g, side):
+    """The grid form's waits for partials and, in the diagnostic's second run, for
+    rows of z alone end in B3G_ERR_TIMEOUT, and the next step is that of a cloth
+    that never met one."""
+    import ctypes as C
+
+    scene = b3g.plain_scene(side)
+    ends = []
+    for waits in (True, False):
+        cloth = b3g.Cloth(scene.mesh, scene.cdef).setup(scene, b3g.SolverOptions.relative(1e-4, 50))
+        cloth.set_cg_strategy(True)
+        if waits:
+            res = C.c_int(0)
+            b3g.check(b3g.lib().b3g_debug_cg_barrier_timeout(cloth.h, 2000, C.byref(res)), "timeout diag")
+            assert res.value == 7  # B3G_ERR_TIMEOUT
+        assert cloth.step(scene.dt)["iterations"] > 0
+        ends.append(cloth.state()["dv"])
+    assert np.array_equal(ends[0], ends[1])
