@@ -77,9 +77,17 @@ static int check_sizes()
     return 0;
 }
 
+// Systems that the tests of the cooperative kernels rely on: not solved on chip.
+static int check_refused()
+{
+    const ResSystem hub{1201, 41u * 1216u, 41, 1200, 0, 0};  // a row of 41 blocks
+    if (resident_shape_on(hub, 148).ctas) return fail("on chip after all", hub, ResShape(), 0);
+    return 0;
+}
+
 // A grid of rows x side vertices, its triangles' couplings; closed: the last
 // row is coupled to the first one; shuffled: in random numbering.
-static int check_mesh(uint32_t rows, uint32_t side, bool closed, bool shuffled)
+static int check_mesh(uint32_t rows, uint32_t side, bool closed, bool shuffled, bool refused = false)
 {
     const uint32_t n = rows * side;
     std::vector<uint32_t> id(n);
@@ -104,6 +112,7 @@ static int check_mesh(uint32_t rows, uint32_t side, bool closed, bool shuffled)
         for (uint32_t j : nb[i]) f(j);
     });
     const ResShape s = resident_shape_on(c, 148);
+    if (refused) return s.ctas ? fail("on chip after all", c, s, 0) : 0;
     if (!s.ctas) return 0;
     if (check_by_band(c, s)) return 1;
     for (uint32_t k = 0; k < s.ctas && s.listed; ++k) {
@@ -122,7 +131,9 @@ static int check_mesh(uint32_t rows, uint32_t side, bool closed, bool shuffled)
 
 int main()
 {
-    if (check_sizes()) return 1;
+    if (check_sizes() || check_refused()) return 1;
+    for (uint32_t side : {240u, 268u, 300u})
+        if (check_mesh(side, side, false, true, true)) return 1;
     const uint32_t sides[][2] = {{27, 27}, {33, 32}, {46, 46}, {34, 34}, {40, 40}, {48, 48}, {64, 64}, {91, 91}, {200, 128}};
     for (const auto& s : sides)
         for (int form = 0; form < 4; ++form)
