@@ -44,7 +44,7 @@ def parse():
     ap.add_argument("--side", type=int, default=256)
     ap.add_argument("--cg", choices=["fused", "persistent"], default="persistent",
                     help="the headline cloth's CG: one persistent launch with one grid reduction per "
-                         "iteration (fused) or two")
+                         "iteration (fused) or two; a cloth that fits on chip is solved there either way")
     ap.add_argument("--assembly", choices=["records", "rows"], default="records",
                     help="how every cloth's system is assembled: each element evaluated once into a record "
                          "(records) or recomputed by each of its rows in two passes (rows); same floats")
@@ -141,21 +141,23 @@ def peaks():
 # DRAM bytes (read + write) of one persistent-CG launch, by (cloth side, CG
 # form): (bytes of one captured launch, that launch's CG iterations), from
 # one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum).
-# * 256 x 256: the whole system stays in L2 after its first touch, so the
-#   figure holds for any iteration count (None).
+# * 256 x 256: on chip; the system is read once, so the figure holds for any
+#   iteration count (None).
 # * 1024 x 1024: the 293 MB system streams from HBM once at the start (A x0)
 #   and once per iteration, so the traffic scales with 1 + iterations (the
 #   captured launch, the third step from rest, ran 10 iterations).
 # Sizes and forms without a capture report null.
 GRID_CG_TRAFFIC = {
-    (256, "persistent"): (36547000, None),
-    (1024, "persistent"): (4107670528 + 631533568, 10),
-    (1024, "fused"): (3919580160 + 676790272, 10),
+    (256, "persistent"): (36538368 + 7424, None),
+    (1024, "persistent"): (4189886976 + 631389440, 10),
+    (1024, "fused"): (3938919936 + 665706496, 10),
 }
-# DRAM bytes over algorithmic bytes of the batched CG launch (512 cloths):
-# 19.46 GB of DRAM traffic against 20.48 GB algorithmic (the average of the
-# run's two timed launches; the captured launch is the second).
-BATCH_CG_TRAFFIC_RATIO = (16734817024 + 2720797440) / 20483036026.0
+# DRAM bytes of the batched CG, by (cloths, cluster): four launches of 15 to 38
+# iterations a cloth each, 1.09 GB every time, since every system is held on chip.
+BATCH_CG_TRAFFIC = {(512, 8): 1007668096 + 83424000}
+# Most vertices of a grid cloth that the persistent strategies solve on chip
+# (k_resident_grid): two rows a thread, 512 threads a CTA, 148 CTAs.
+ON_CHIP_VERTICES = 2 * 512 * 148
 
 
 def grid_cg_traffic(side: int, form: str, iterations: float):
@@ -180,8 +182,12 @@ def algorithmic_bytes(info: dict, kernel: str) -> float:
         return (3 * 12 + 12 + 1) * n
     if kernel == "cg_init":
         return 40.0 * blocks + (12 * 3 + 1 + 3 * 12) * n
+    if kernel == "resident_cg":
+        # the whole solve on chip: the start of the solve below; what the
+        # iterations move stays in shared memory and L2
+        return 40.0 * blocks + 73.0 * n
     if kernel.startswith("grid_cg"):
-        # the whole persistent solve: the start (A x0: A once, m_x, b, P^-1
+        # the whole solve by a kernel that reads its system in every iteration: the start (A x0: A once, m_x, b, P^-1
         # read, r and z written, filter byte), then per iteration the MPCG's
         # minimum, whatever the form: A values and columns once (40 B per
         # block), the row pointer (4 B per row), the direction read and the
@@ -243,7 +249,7 @@ def run_ours(args, rank, world):
     scene = b3g.sphere_scene(args.side, seed=2 + rank)
     opts = b3g.SolverOptions.relative(1e-4, 200, b3g.DOT_F64)
     cloth = b3g.Cloth(scene.mesh, scene.cdef, device=dev).setup(scene, opts)
-    # the whole solve in one persistent cooperative launch
+    # the whole solve in one persistent launch, on chip where it fits
     cloth.set_cg_strategy(True, fused=args.cg == "fused")
     cloth.set_assembly(args.assembly)
     info = cloth.info()
@@ -323,12 +329,13 @@ def run_ours(args, rank, world):
         # one persistent launch per step holds the whole CG
         kern.pop("cg_update")
         kern.pop("cg_direction")
-        kern["grid_cg"] = kern.pop("cg_spmv")
-        kern["grid_cg"] = (kern["grid_cg"][0], len(prof))
+        kern["resident_cg" if n <= ON_CHIP_VERTICES else "grid_cg"] = (kern.pop("cg_spmv")[0], len(prof))
     total = sum(v[0] for v in kern.values())
     dom = max(kern, key=lambda k: kern[k][0])
     avg_ms = kern[dom][0] / kern[dom][1]
-    alg = algorithmic_bytes(info, dom if dom != "grid_cg" else f"grid_cg:{it_total / len(prof)}")
+    solve = dom in ("resident_cg", "grid_cg")
+    streamed = algorithmic_bytes(info, f"grid_cg:{it_total / len(prof)}") if solve else None
+    alg = streamed if dom == "grid_cg" else algorithmic_bytes(info, dom)
     peak, peak_kind = peaks()
     achieved = alg / (avg_ms / 1000.0) / 1e9
     # the assembly (both of its launches) against the same roofline
@@ -342,12 +349,18 @@ def run_ours(args, rank, world):
         "value": value, "ms_per_step": 1000.0 * dev_s / args.steps, "wall_s": wall, "e2e": e2e, "fp64": fp64,
         "iterations_mean": float(np.mean(iters)), "active_contacts_mean": float(np.mean(contacts)),
         "launches": launches, "clocks": clocks.summary(), "info": info,
-        "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "peak_kind": peak_kind,
+        # on chip the system is read once: HBM is no bound there, two grid
+        # reductions an iteration are.  streamed_*: what a CG that reads its
+        # system in every iteration would move in that time.
+        "roofline": {"bound": "latency of the grid reductions" if dom == "resident_cg" else "hbm", "kernel": dom,
+                     "achieved": achieved, "peak": peak, "peak_kind": peak_kind,
                      "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": (grid_cg_traffic(args.side, args.cg, it_total / len(prof))
-                                 if dom == "grid_cg" else None),
+                     "us_per_cg_iteration": 1e3 * kern[dom][0] / max(it_total, 1) if solve else None,
+                     "traffic": grid_cg_traffic(args.side, args.cg, it_total / len(prof)) if solve else None,
                      "traffic_source": "ncu capture of one launch at this size",
-                     "algorithmic_bytes_per_launch": alg, "avg_launch_ms": avg_ms,
+                     "algorithmic_bytes_per_launch": alg, "streamed_bytes_per_launch": streamed,
+                     "streamed_frac": streamed / (avg_ms / 1000.0) / 1e9 / peak if solve else None,
+                     "avg_launch_ms": avg_ms,
                      "share": kern[dom][0] / total if total else None},
         "kernel_ms": {k: v[0] / v[1] for k, v in kern.items()},
         "assembly": assembly,
@@ -438,6 +451,8 @@ def run_batched(args, dev: int, cpu_sample: bool = False):
     blocks = np.array([c.info()["blocks"] for c in cloths], dtype=np.float64)
     nrows = np.array([c.n for c in cloths], dtype=np.float64)
     ms, cg_ms, iters, cg_bytes = [], [], [], []
+    traffic = BATCH_CG_TRAFFIC.get((len(scenes), int(sched["cluster"])))
+    once = float(np.sum(40.0 * blocks + 73.0 * nrows))  # every system read once, its vectors read and written
     launches0 = b3g.kernel_launch_count()
     for _ in range(args.batch_steps):
         out = batch.step(cloths, dt, per_cloth=True)
@@ -445,7 +460,7 @@ def run_batched(args, dev: int, cpu_sample: bool = False):
         cg_ms.append(out["cg_ms"])
         iters.append(out["cg_iterations_total"] / out["count"])
         it = np.array([pc["iterations"] for pc in out["per_cloth"]], dtype=np.float64)
-        # the same per-cloth count as the persistent single-cloth solve
+        # if every cloth read its system in every iteration
         cg_bytes.append(float(np.sum(40.0 * blocks + 73.0 * nrows + it * (40.0 * blocks + 146.0 * nrows))))
     launches = b3g.kernel_launch_count() - launches0
     batched = replicas.aggregate_rate(rows * len(ms), sum(ms) / 1000.0)
@@ -484,14 +499,19 @@ def run_batched(args, dev: int, cpu_sample: bool = False):
             "schedule": {"cluster": sched["cluster"],
                          "split_size_classes": [k for k, v in enumerate(sched["split_class"]) if v]},
             "gpu_launches": launches, "steps": len(ms),
-            "roofline": {"bound": "hbm", "kernel": "batch_cg", "achieved": sum(cg_bytes) / (sum(cg_ms) / 1e3) / 1e9,
+            # on clusters of 8 every cloth is solved on chip and reads its
+            # system once (smaller clusters leave the largest to batch_cg);
+            # streamed_*: if all read it in every iteration
+            "roofline": {"bound": "latency of the teams' reductions",
+                         "kernel": "batch_resident" if sched["cluster"] == 8 else "batch_resident and batch_cg",
+                         "achieved": once * len(cg_ms) / (sum(cg_ms) / 1e3) / 1e9,
                          "peak": peaks()[0], "peak_kind": peaks()[1], "unit": "GB/s",
-                         "frac": sum(cg_bytes) / (sum(cg_ms) / 1e3) / 1e9 / peaks()[0],
-                         "algorithmic_bytes_per_launch": sum(cg_bytes) / len(cg_bytes),
-                         "traffic": BATCH_CG_TRAFFIC_RATIO * sum(cg_bytes) / len(cg_bytes),
-                         "traffic_source": "DRAM/algorithmic ratio of one captured 512-cloth launch",
-                         "dram_frac": (BATCH_CG_TRAFFIC_RATIO * sum(cg_bytes) / (sum(cg_ms) / 1e3) / 1e9
-                                       / peaks()[0]),
+                         "frac": once * len(cg_ms) / (sum(cg_ms) / 1e3) / 1e9 / peaks()[0],
+                         "algorithmic_bytes_per_launch": once,
+                         "streamed_bytes_per_launch": sum(cg_bytes) / len(cg_bytes),
+                         "streamed_frac": sum(cg_bytes) / (sum(cg_ms) / 1e3) / 1e9 / peaks()[0],
+                         "traffic": traffic, "traffic_source": "ncu captures of this size's launch",
+                         "dram_frac": traffic / (sum(cg_ms) / len(cg_ms) / 1e3) / 1e9 / peaks()[0] if traffic else None,
                          "avg_launch_ms": sum(cg_ms) / len(cg_ms), "share": sum(cg_ms) / sum(ms)},
             "l2": "inputs larger than L2 (about 1 GB of resident cloth state)",
             "cpu_baseline": cpu_batch_baseline(args.batch_count) if cpu_sample else None}
@@ -544,7 +564,7 @@ def run_softbody(args, dev: int, cpu_sample: bool):
                          "algorithmic_bytes_per_step": step_bytes}
     out = {"workload": f"block{side}x{side}x{side}_pinned", "nodes": n, "tetrahedra": t, "blocks": nnz,
            "cg": "reference rule (20 iterations, f32 dots)",
-           "cg_strategy": "persistent cooperative launch (the default)"}
+           "cg_strategy": "one persistent launch (the default)"}
     out.update(by["persistent"])
     out["by_strategy"] = by
     if cpu_sample:
@@ -628,8 +648,10 @@ def run_self_collision(args, dev: int, cpu_sample: bool):
     scene = b3g.self_collision_scene(args.self_side)
     lo, hi = 60, 120
     # warm-up: one untimed pass of the same 120 steps on another cloth, so
-    # that first-use costs (module loading, the contact list's first growth
-    # to this scene's size) stay out of the timed steps
+    # that first-use costs (module loading) stay out of the timed steps.  The
+    # timed cloth's contact list still grows in them, twice at 24 x 24: a step
+    # that outgrows the list makes its buffers anew, which takes from a
+    # fraction of a millisecond to several.
     warm = b3g.Cloth(scene.mesh, scene.cdef, device=dev).setup(scene)
     warm.set_cg_strategy(True)
     for _ in range(hi):
@@ -653,6 +675,8 @@ def run_self_collision(args, dev: int, cpu_sample: bool):
     out = {"workload": f"grid{args.self_side}_self_collision_capsule", "vertices": n,
            "triangles": scene.mesh.triangle_count, "steps": f"{lo}-{hi - 1}",
            "ms_per_step": sum(ms) / len(ms), "ms_median": float(np.median(ms)), "ms_max": float(max(ms)),
+           "slowest_step": {"step": lo + int(np.argmax(ms)), "contacts": contacts[int(np.argmax(ms))],
+                            "active": active[int(np.argmax(ms))], "levels": levels[int(np.argmax(ms))]},
            "vertex_steps_per_s": n * len(ms) / (sum(ms) / 1e3),
            "tri_contacts_mean": float(np.mean(contacts)), "active_mean": float(np.mean(active)),
            "active_max": int(max(active)), "levels_mean": float(np.mean(levels)), "gpu_launches": launches}
@@ -952,7 +976,9 @@ def main():
         "config": {"workload": f"grid{args.side}x{args.side}_bending_sphere", "vertices": n,
                    "triangles": r["info"]["triangles"], "springs": r["info"]["springs"],
                    "blocks": r["info"]["blocks"], "cg": "relative residual 1e-4, max 200, fp64 dots",
-                   "cg_strategy": ("persistent cooperative launch, one grid reduction per iteration"
+                   "cg_strategy": ("one cooperative launch, the system on chip, two grid reductions per iteration"
+                                   if n <= ON_CHIP_VERTICES else
+                                   "persistent cooperative launch, one grid reduction per iteration"
                                    if args.cg == "fused" else "persistent cooperative launch, two grid "
                                                               "reductions per iteration"),
                    "contact_iterations": [8, 2], "parallelism": f"replicas{world}",

@@ -42,3 +42,9 @@ def test_summary_repeats_section_figures():
     assert s["headline_vertex_steps_per_s"] == 5.5e7 and s["headline_e2e"] == 4.9e7
     assert s["assembly_ms"] == 0.083 and s["assembly_frac"] == 0.095
     assert s["batched_speedup_vs_plain"] == 7.3 and s["serving_vertex_steps_per_s"] is None
+
+
+def test_on_chip_cg_bytes_model():
+    # the system and its vectors once, whatever the iterations
+    assert bench.algorithmic_bytes(INFO, "resident_cg") == bench.algorithmic_bytes(INFO, "grid_cg:0")
+    assert abs(bench.grid_cg_traffic(256, "persistent", 100) / bench.algorithmic_bytes(INFO, "resident_cg") - 1.0) < 0.1
