@@ -939,9 +939,10 @@ class SoftBody:
         check(lib().b3g_softbody_set_solver(self.h, C.byref(c)), "softbody_set_solver")
 
     def set_cg_strategy(self, persistent: bool, fused: bool = False) -> None:
-        """True (the default): the MPCG as one persistent cooperative launch
-        (fused: one grid reduction per iteration); False: three launches per
-        CG iteration."""
+        """True (the default): the MPCG in one launch, on chip where the body
+        fits (b3g.h), else as a persistent cooperative launch (fused: with one
+        grid reduction per iteration); False: three launches per CG
+        iteration."""
         code = 0 if not persistent else 2 if fused else 1
         check(lib().b3g_softbody_set_cg_strategy(self.h, code), "softbody_set_cg_strategy")
 

@@ -1,5 +1,5 @@
 // The MPCG of one cloth with its system held on chip: device code shared by
-// the single-cloth launches (resident_cg.cu) and the batch (batch_cg.cu).
+// the single-cloth launches (resident_cg.cu) and the batch (batch_resident.cu).
 //
 // A team of CTAs owns the cloth's rows in contiguous chunks, at most RPT rows
 // a thread.  For the whole solve a CTA keeps in shared memory

@@ -86,7 +86,9 @@ struct ResShape {
 };
 
 // CTAs of a system of n rows on one cluster, and its rows a CTA there or on
-// the grid of a 148-SM device.
+// the grid of a 148-SM device, a B200's.  (Halos are counted for that grid, when
+// a cloth is laid out; with another number of SMs a system whose band is too
+// wide is left to the cooperative kernels.)
 inline uint32_t resident_team(uint32_t n)
 {
     if (n > (uint32_t)(kResMaxTeam * kResMaxThreads)) return 0u;

@@ -1105,8 +1105,11 @@ b3g_status b3g_softbody_create(uint32_t vertex_count, const float* vertices, uin
     uint32_t* asm_nodes = (uint32_t*)take((size_t)n * 4);
     d.asm_nodes = asm_nodes;
     // three launches by the lanes a node needs; a body of few nodes leaves the
-    // GPU idle anyway and takes one (512 nodes: 138 us a step against 143,
-    // 9,261: 206 against 202)
+    // GPU idle anyway and takes one.  A step in us, one launch and three: 512
+    // nodes 131 and 149, 4,096 228 and 235, 8,000 204 and 209, 9,261 205 and
+    // 209, 12,167 220 and 225, 15,625 239 and 234; of 68,921 the assembly
+    // alone 209 and 170.  So the two cross near 14,000 nodes, and from the line
+    // to there three launches cost two hundredths.
     std::vector<uint32_t> by_lanes;
     by_lanes.reserve(n);
     for (int cls = 0; cls < 3; ++cls) {

@@ -270,15 +270,18 @@ b3g_status b3g_cloth_step(b3g_cloth* cloth, float dt, uint32_t velocity_iteratio
                           uint32_t position_iterations, b3g_step_stats* stats);
 
 /* How one cloth's CG runs on the GPU.  A cloth whose system fits on chip
- * (rows of at most 16 blocks, couplings within a band of vertex numbers that
- * a CTA can hold) is solved there in one launch, with the same arithmetic: up
- * to 4,096 vertices by one CTA or cluster under every strategy, up to about
- * 150,000 by a cooperative launch under the persistent ones (bounded waits,
- * B3G_ERR_TIMEOUT if one gives up).  Otherwise: LAUNCHES (default): three
- * kernels per iteration inside a CUDA-graph while loop.  PERSISTENT: one
+ * is solved there in one launch, with the same arithmetic: up to 4,096 vertices
+ * by one CTA or cluster under every strategy, up to about 150,000 by a
+ * cooperative launch under the persistent ones (bounded waits, B3G_ERR_TIMEOUT
+ * if one gives up).  It fits if its rows have at most 32 blocks (16 above about
+ * 75,000 vertices), half of the blocks find room in shared memory, and the
+ * vertices outside a CTA's own that its rows couple to are at most 2,048:
+ * those within the band of vertex numbers that the couplings span, or, where
+ * that band holds more, those that the rows name.  Otherwise: LAUNCHES (default):
+ * three kernels per iteration inside a CUDA-graph while loop.  PERSISTENT: one
  * cooperative launch for the whole solve, two grid reductions per iteration,
- * separated by grid barriers with bounded waits; for large cloths.  PERSISTENT_FUSED: as PERSISTENT with one grid reduction per
- * iteration.  Each vertex publishes r, s and p once per iteration, and every
+ * separated by grid barriers with bounded waits; for large cloths.
+ * PERSISTENT_FUSED: as PERSISTENT with one grid reduction per iteration.  Each vertex publishes r, s and p once per iteration, and every
  * row forms its neighbours' next direction from them.  The reduction returns
  * p.s, s.z, s.P^-1 s and r.z (z = S P^-1 r) of the iterate: alpha = r.z / p.s
  * as the reference's, and the next r.z expanded as
@@ -596,10 +599,12 @@ b3g_status b3g_softbody_set_velocity(b3g_softbody* body, uint32_t node, const fl
 b3g_status b3g_softbody_set_position(b3g_softbody* body, uint32_t node, const float* position);
 /* Default: the reference's MPCG (20 iterations, FLT_EPSILON^2, FP32 dots). */
 b3g_status b3g_softbody_set_solver(b3g_softbody* body, const b3g_solver_opts* opts);
-/* How the MPCG runs: B3G_CG_PERSISTENT (the default) is one cooperative
- * launch per solve with two grid reductions per iteration, on a copy of the
- * system in the cloth's SELL-32 layout with its rows ordered by degree;
- * B3G_CG_PERSISTENT_FUSED the same with one grid reduction per iteration;
+/* How the MPCG runs: B3G_CG_PERSISTENT (the default) is one launch per solve,
+ * on a copy of the system in the cloth's SELL-32 layout with its rows ordered
+ * by degree: on chip where it fits (b3g_cloth_set_cg_strategy), else a
+ * cooperative launch with two grid reductions per iteration;
+ * B3G_CG_PERSISTENT_FUSED the same with one grid reduction per iteration in
+ * the cooperative launch (a body that fits is solved on chip as above);
  * B3G_CG_LAUNCHES three launches per iteration on the block-CSR system.
  * All solve the same system by the same rule; their dot products sum in
  * different orders. */
