@@ -326,7 +326,7 @@ typedef struct {
     float contacts_update_ms;
     float assemble_ms;
     float cg_init_ms;
-    float cg_spmv_ms;       /* all iterations */
+    float cg_spmv_ms;       /* all iterations; the whole CG where it is one launch */
     float cg_update_ms;     /* all iterations */
     float cg_direction_ms;  /* all iterations */
     float finalize_ms;
